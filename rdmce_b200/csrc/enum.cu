@@ -1916,11 +1916,30 @@ __device__ __forceinline__ void gen_solve(const Ctx &c, const Gen &G, uint32_t r
 
 // ------------------------------------------------------------ root build
 
-// C = N(v0) & N(v1) (sorted) into cand[]; |C|, or 0xffffffff beyond cap
-__device__ uint32_t intersect(const DevGraph &g, uint32_t v0, uint32_t v1, uint32_t *cand, uint64_t cap) {
-  const uint32_t lane = lane_id();
-  const uint32_t *a = g.adj + g.off[v0], *b = g.adj + g.off[v1];
-  uint32_t da = g.off[v0 + 1] - g.off[v0], db = g.off[v1 + 1] - g.off[v1];
+// Which of four sorted values per lane occur in the sorted list b[0..n), as
+// four branchless binary searches in step: n is warp-uniform, so every lane
+// runs the same trip count and the four dependent load chains overlap.
+__device__ __forceinline__ void contains4(const uint32_t *b, uint32_t n, const uint32_t (&val)[4], bool (&hit)[4]) {
+  uint32_t pos[4] = {0, 0, 0, 0};
+  uint32_t len = n;
+  while (len > 1) {
+    const uint32_t half = len >> 1;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (__ldg(b + pos[k] + half - 1) < val[k]) pos[k] += half;
+    len -= half;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) hit[k] = n && __ldg(b + pos[k]) == val[k];
+}
+
+// The shorter of two adjacency lists in (a, da), the longer in (b, db).
+__device__ __forceinline__ void shorter_first(const DevGraph &g, uint32_t v0, uint32_t v1, const uint32_t *&a,
+                                              uint32_t &da, const uint32_t *&b, uint32_t &db) {
+  a = g.adj + g.off[v0];
+  b = g.adj + g.off[v1];
+  da = g.off[v0 + 1] - g.off[v0];
+  db = g.off[v1 + 1] - g.off[v1];
   if (da > db) {
     const uint32_t *t = a;
     a = b;
@@ -1929,15 +1948,34 @@ __device__ uint32_t intersect(const DevGraph &g, uint32_t v0, uint32_t v1, uint3
     da = db;
     db = td;
   }
+}
+
+// C = N(v0) & N(v1) (sorted) into cand[]; |C|, or 0xffffffff beyond cap.
+// Bound by the latency of the searches in the longer list, so four of the
+// shorter list's 32-element groups are searched at a time.
+__device__ uint32_t intersect(const DevGraph &g, uint32_t v0, uint32_t v1, uint32_t *cand, uint64_t cap) {
+  const uint32_t lane = lane_id();
+  const uint32_t *a, *b;
+  uint32_t da, db;
+  shorter_first(g, v0, v1, a, da, b, db);
   uint32_t nc = 0;
-  for (uint32_t base = 0; base < da; base += 32) {
-    const uint32_t t = base + lane;
-    const uint32_t val = t < da ? __ldg(a + t) : 0;
-    const bool hit = t < da && contains_u32(b, db, val);
-    const uint32_t bal = __ballot_sync(kFull, hit);
-    if (nc + __popc(bal) > cap) return 0xffffffffu;
-    if (hit) cand[nc + __popc(bal & lanemask_lt())] = val;
-    nc += __popc(bal);
+  for (uint32_t base = 0; base < da; base += 128) {
+    uint32_t val[4];
+    bool hit[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t t = base + 32 * k + lane;
+      val[k] = t < da ? __ldg(a + t) : 0;
+    }
+    contains4(b, db, val, hit);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      hit[k] = hit[k] && base + 32 * k + lane < da;
+      const uint32_t bal = __ballot_sync(kFull, hit[k]);
+      if (nc + __popc(bal) > cap) return 0xffffffffu;
+      if (hit[k]) cand[nc + __popc(bal & lanemask_lt())] = val[k];
+      nc += __popc(bal);
+    }
   }
   __syncwarp();
   return nc;
@@ -1947,16 +1985,9 @@ __device__ uint32_t intersect(const DevGraph &g, uint32_t v0, uint32_t v1, uint3
 // sizes the large-scratch pass for a root whose ego network overflowed the slab.
 __device__ void intersect_count(const DevGraph &g, uint32_t v0, uint32_t v1, uint32_t *nc_out, uint32_t *nx_out) {
   const uint32_t lane = lane_id();
-  const uint32_t *a = g.adj + g.off[v0], *b = g.adj + g.off[v1];
-  uint32_t da = g.off[v0 + 1] - g.off[v0], db = g.off[v1 + 1] - g.off[v1];
-  if (da > db) {
-    const uint32_t *t = a;
-    a = b;
-    b = t;
-    const uint32_t td = da;
-    da = db;
-    db = td;
-  }
+  const uint32_t *a, *b;
+  uint32_t da, db;
+  shorter_first(g, v0, v1, a, da, b, db);
   uint32_t nc = 0, nx = 0;
   for (uint32_t base = 0; base < da; base += 32) {
     const uint32_t t = base + lane;
@@ -1969,9 +2000,166 @@ __device__ void intersect_count(const DevGraph &g, uint32_t v0, uint32_t v1, uin
   *nx_out = nx;
 }
 
-// Ego bitmap rows (candidate rows, then X rows with a candidate neighbour).
+// Scratch of the root build: the candidates P and the rows in flight.  It
+// overlays per-warp state that only a running solve uses.
+struct BuildScratch {
+  uint32_t P[256];     // candidates, padded to a power of two with 0xffffffff (p <= 256)
+  uint32_t obase[32];  // non-empty row o of the batch: element t of the flattened lists is adj[obase[o] + t]
+  uint32_t orow[32];   // its row in the batch
+};
+static_assert(offsetof(WarpSmem, t0_s1) - offsetof(WarpSmem, t0f) >= sizeof(BuildScratch),
+              "the build scratch fits over the 32-bit tier's frames and exchange buffer");
+
+// First index whose value is >= key in a sorted list in the warp's slab
+// (written by this kernel, so read with ordinary loads).
+__device__ __forceinline__ uint32_t slab_lower_bound(const uint32_t *a, uint32_t n, uint32_t key) {
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (a[mid] < key) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// The only j < p at which P[j] can be y, over the candidates in shared memory
+// (padded) or in the slab.
+__device__ __forceinline__ uint32_t find_cand(const BuildScratch *bs, uint32_t top, const uint32_t *Pl, uint32_t p,
+                                              uint32_t y) {
+  if (top == 0) return slab_lower_bound(Pl, p, y);
+  uint32_t pos = 0;
+  for (uint32_t s = top; s; s >>= 1)
+    if (bs->P[pos + s - 1] < y) pos += s;
+  return pos;
+}
+
+// Ego bitmap rows (candidate rows, then X rows with a candidate neighbour), up
+// to 4096 candidates.
+//
+// A row of member u is N(u) & P.  One row at a time leaves the warp waiting on
+// two binary searches and a few loads for each row, so rows are built in
+// batches of up to 32 (64 words of bitmap): every lane finds the part of one
+// member's list that spans P -- most X members have no neighbour above v1 and
+// end there -- and the parts are read as one flattened list, 32 neighbouring
+// elements at a time whatever the rows' lengths.  An element's row comes from
+// the row starts inside the window (one OR-reduction), its column from a
+// search in shared memory.  A part much longer than P is probed for the
+// candidates instead.
+// Measured (B200), against a row at a time: Chung-Lu 10^4 1.07 -> 0.28 ms (the
+// longest root 1.9e6 -> 0.28e6 cycles); planted cliques of 40-200 vertices in
+// 10^5, edge roots only (99 % of the time is this build) 297 -> 202 ms.
 __device__ uint32_t build_rows(const DevGraph &g, const uint32_t *cand, uint32_t x, uint32_t p, uint32_t W,
-                               uint64_t *rows, uint64_t *rowbuf) {
+                               uint64_t *rows, WarpSmem *sm) {
+  const uint32_t lane = lane_id();
+  const uint32_t *Pl = cand + x;
+  BuildScratch *bs = (BuildScratch *)sm->t0f;
+  uint64_t *acc = sm->rowbuf;  // rows of the batch, W words each
+  uint32_t *acc32 = (uint32_t *)acc;
+  const uint32_t pmin = Pl[0], pmax = Pl[p - 1];
+  // top: first step of the column search, a power of two with 2 * top >= p (0: search the slab)
+  uint32_t top = 0;
+  if (p <= 256) {
+    top = p <= 2 ? 1u : 1u << (31 - __clz(p - 1));
+    for (uint32_t i = lane; i < 2 * top; i += 32) bs->P[i] = i < p ? Pl[i] : 0xffffffffu;
+  }
+  const uint32_t nb = min(32u, 64u / W);
+  uint32_t nrows = 0;
+  for (uint32_t mb = 0; mb < p + x; mb += nb) {
+    const uint32_t m = mb + lane;
+    const bool mine = lane < nb && m < p + x;
+    uint32_t lo = 0, len = 0;
+    if (mine) {
+      const uint32_t u = m < p ? Pl[m] : cand[m - p];
+      const uint32_t b = g.off[u], e = g.off[u + 1];
+      if (__ldg(g.adj + e - 1) >= pmin) {
+        lo = b + lower_bound_u32(g.adj + b, e - b, pmin);
+        len = lower_bound_u32(g.adj + lo, e - lo, pmax + 1);
+      }
+    }
+    for (uint32_t w = lane; w < nb * W; w += 32) acc[w] = 0;
+    // probing costs p searches of a warp's lanes, reading the part len / 32 loads
+    const bool probe = len > 8 * p + 64;
+    const uint32_t sl = probe ? 0 : len;
+    uint32_t incl = sl;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, incl, d);
+      if (lane >= (uint32_t)d) incl += y;
+    }
+    const uint32_t T = __shfl_sync(kFull, incl, 31), first = incl - sl;
+    const uint32_t ne = __ballot_sync(kFull, sl != 0);
+    if (sl) {
+      const uint32_t o = __popc(ne & lanemask_lt());
+      bs->obase[o] = lo - first;
+      bs->orow[o] = lane;
+    }
+    __syncwarp();
+    // window t0: row starts inside it, and this lane's element and its row
+    uint32_t started = 0, heads = 0, row = 0, y = 0;
+    auto fetch = [&](uint32_t t0) {
+      heads = __reduce_or_sync(kFull, sl && first - t0 < 32 ? 1u << (first - t0) : 0u);
+      const uint32_t o = started + __popc(heads & (lanemask_lt() | (1u << lane))) - 1;
+      started += __popc(heads);
+      row = bs->orow[o];
+      y = t0 + lane < T ? __ldg(g.adj + (bs->obase[o] + t0 + lane)) : 0;
+    };
+    if (T) fetch(0);
+    for (uint32_t t0 = 0; t0 < T; t0 += 32) {
+      const uint32_t nheads = __popc(heads), yc = y;
+      const uint32_t rowkey = row * 2 * W;
+      const bool in = t0 + lane < T;
+      if (t0 + 32 < T) fetch(t0 + 32);  // the next window's loads run under this one's search
+      const uint32_t j = find_cand(bs, top, Pl, p, yc);
+      const bool hit = in && j < p && (top ? bs->P[j] : Pl[j]) == yc;
+      const uint32_t key = rowkey + (j >> 5);
+      const uint32_t bit = 1u << (j & 31);
+      uint32_t rem = __ballot_sync(kFull, hit);
+      if (__popc(rem) <= 8 || nheads > 2) {
+        if (hit) atomicOr(&acc32[key], bit);
+      } else {
+        // long rows with many hits: neighbouring elements share a word, and
+        // atomics on one word would run one after another
+        while (rem) {
+          const uint32_t l = __ffs(rem) - 1;
+          const uint32_t kl = __shfl_sync(kFull, key, l);
+          const bool same = hit && key == kl;
+          const uint32_t bits = __reduce_or_sync(kFull, same ? bit : 0u);
+          if (lane == l) acc32[key] |= bits;
+          rem &= ~__ballot_sync(kFull, same);
+        }
+      }
+      __syncwarp();
+    }
+    for (uint32_t pr = __ballot_sync(kFull, probe); pr; pr &= pr - 1) {
+      const uint32_t l = __ffs(pr) - 1;
+      const uint32_t *part = g.adj + __shfl_sync(kFull, lo, l);
+      const uint32_t n = __shfl_sync(kFull, len, l);
+      for (uint32_t base = 0; base < p; base += 32) {
+        const uint32_t j = base + lane;
+        const uint32_t bal = __ballot_sync(kFull, j < p && contains_u32(part, n, Pl[j]));
+        if (lane == 0) acc32[l * 2 * W + (base >> 5)] = bal;
+      }
+    }
+    __syncwarp();
+    uint64_t any = 0;
+    if (mine)
+      for (uint32_t w = 0; w < W; w++) any |= acc[lane * W + w];
+    const bool keep = mine && (m < p || any);
+    const uint32_t bal = __ballot_sync(kFull, keep);
+    if (keep) {
+      uint64_t *row = rows + (uint64_t)(nrows + __popc(bal & lanemask_lt())) * W;
+      for (uint32_t w = 0; w < W; w++) row[w] = acc[lane * W + w];
+    }
+    nrows += __popc(bal);
+    __syncwarp();
+  }
+  return nrows;
+}
+
+// The same for more than 4096 candidates: one row at a time, probed for the
+// candidates.
+__device__ uint32_t build_rows_wide(const DevGraph &g, const uint32_t *cand, uint32_t x, uint32_t p, uint32_t W,
+                                    uint64_t *rows) {
   const uint32_t lane = lane_id();
   const uint32_t *Pl = cand + x;
   const uint32_t pmin = Pl[0], pmax = Pl[p - 1];
@@ -1988,41 +2176,22 @@ __device__ uint32_t build_rows(const DevGraph &g, const uint32_t *cand, uint32_t
     }
     lo = __shfl_sync(kFull, lo, 0);
     hi = __shfl_sync(kFull, hi, 0);
-    bool any;
-    if (hi - lo < p && W <= 64) {
-      for (uint32_t w = lane; w < W; w += 32) rowbuf[w] = 0;
-      __syncwarp();
-      bool hit = false;
-      for (uint32_t e = lo + lane; e < hi; e += 32) {
-        const uint32_t y = __ldg(nu + e);
-        const uint32_t j = lower_bound_u32(Pl, p, y);
-        if (j < p && Pl[j] == y) {
-          atomicOr((unsigned long long *)&rowbuf[j >> 6], 1ULL << (j & 63));
-          hit = true;
-        }
+    uint64_t word = 0;
+    bool any = false;
+    const uint32_t *sl = nu + lo;
+    const uint32_t sn = hi - lo;
+    for (uint32_t base = 0; base < p; base += 32) {
+      const uint32_t j = base + lane;
+      const bool hit = j < p && contains_u32(sl, sn, Pl[j]);
+      const uint32_t bal = __ballot_sync(kFull, hit);
+      any |= bal != 0;
+      if (base & 32) {
+        word |= (uint64_t)bal << 32;
+        if (lane == 0) row[base >> 6] = word;
+      } else {
+        word = bal;
+        if (base + 32 >= p && lane == 0) row[base >> 6] = word;
       }
-      any = __any_sync(kFull, hit);
-      __syncwarp();
-      for (uint32_t w = lane; w < W; w += 32) row[w] = rowbuf[w];
-    } else {
-      uint64_t word = 0;
-      bool hitany = false;
-      const uint32_t *sl = nu + lo;
-      const uint32_t sn = hi - lo;
-      for (uint32_t base = 0; base < p; base += 32) {
-        const uint32_t j = base + lane;
-        const bool hit = j < p && contains_u32(sl, sn, Pl[j]);
-        const uint32_t bal = __ballot_sync(kFull, hit);
-        hitany |= bal != 0;
-        if (base & 32) {
-          word |= (uint64_t)bal << 32;
-          if (lane == 0) row[base >> 6] = word;
-        } else {
-          word = bal;
-          if (base + 32 >= p && lane == 0) row[base >> 6] = word;
-        }
-      }
-      any = hitany;
     }
     __syncwarp();
     if (r < p || any) nrows++;
@@ -2043,7 +2212,7 @@ __device__ bool solve_root(const Ctx &c, uint64_t r) {
     if (c.lane == 0) c.sm->cyc[kCycBuild] += now() - tb0;
     return false;
   }
-  const uint32_t x = nc ? lower_bound_u32(cand, nc, v1) : 0;
+  const uint32_t x = slab_lower_bound(cand, nc, v1);
   const uint32_t p = nc - x;
   const uint64_t s1 = g.h1[v0] + g.h1[v1], s2 = g.h2[v0] + g.h2[v1];
   const uint32_t W = (p + 63) / 64;
@@ -2069,7 +2238,7 @@ __device__ bool solve_root(const Ctx &c, uint64_t r) {
     return true;
   }
   uint64_t *rows = (uint64_t *)(c.slab + L.rows_off);
-  const uint32_t nrows = build_rows(g, cand, x, p, W, rows, c.sm->rowbuf);
+  const uint32_t nrows = W <= 64 ? build_rows(g, cand, x, p, W, rows, c.sm) : build_rows_wide(g, cand, x, p, W, rows);
   __syncwarp();
   if (c.lane == 0) c.sm->cyc[kCycBuild] += now() - tb0;
   if (p <= 32 && nrows <= 32) {
@@ -2398,11 +2567,11 @@ __global__ void k_pool_init(EnumCtl *ctl, uint32_t *free_slot, unsigned long lon
     free_seq[i] = (unsigned long long)i + 1;  // filled for the consumer of position i
     ready_seq[i] = i;                        // free for the producer of position i
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    EnumCtl z{};
-    z.free_tail = n;
-    z.active = 0;
-    *ctl = z;
+  // word by word: the compiler takes minutes over a copy of the padded struct
+  if (blockIdx.x == 0) {
+    for (uint32_t w = threadIdx.x; w < sizeof(EnumCtl) / 4; w += blockDim.x) ((uint32_t *)ctl)[w] = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) ctl->free_tail = n;
   }
 }
 
