@@ -96,6 +96,7 @@ struct DevGraph {
   const uint64_t *h2;       // n: mix64(label ^ golden)
   const uint32_t *root_v0;  // m: roots (v0 < v1) in CSR order
   const uint32_t *root_v1;  // m
+  const uint32_t *root_off; // n + 1: first root of each vertex v0 (its roots are consecutive)
   const uint32_t *slot;     // n or null: result slot of each vertex (batched graphs)
 };
 
@@ -117,7 +118,7 @@ mce_status reduce_max_u32(const uint32_t *in, uint64_t n, uint32_t *d_out, cudaS
 // on demand and kept for reuse (the role of the reference's BufferManager,
 // include/context_gpu.cuh:4-32, without its worst-case sizing).
 struct Scratch {
-  static constexpr int kSlots = 8;
+  static constexpr int kSlots = 9;
   int device = 0;
   // set: buffers are allocated and freed stream-ordered on this stream (no
   // device-wide synchronisation when one grows), for an owner whose work

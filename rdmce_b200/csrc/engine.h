@@ -22,6 +22,7 @@ struct DeviceGraph {
   uint64_t *h2 = nullptr;       // n
   uint32_t *root_v0 = nullptr;  // m
   uint32_t *root_v1 = nullptr;  // m
+  uint32_t *root_off = nullptr; // n + 1: first root of each vertex
   uint32_t *slot = nullptr;     // n, batched mode only
   uint32_t max_degree = 0;
   uint32_t degeneracy = 0;
@@ -143,6 +144,11 @@ struct EnumParams {
   uint64_t n_heavy;                      // entries in heavy_list
   const uint64_t *root_list;             // list mode: root ids (else the range [rb, re))
   uint64_t n_list;                       // entries in root_list
+  int vertex_pass;                       // work items are the vertices of the range, not its roots
+  uint64_t single_items;                 // vertex pass: claims of one vertex; later claims take kVertexChunk
+  uint32_t *edge_out;                    // vertex pass: roots left to the edge pass
+  unsigned int *edge_n;                  // how many
+  const uint32_t *edge_list;             // edge pass: those roots (edge_n of them)
   unsigned long long *next;              // claim counter
   char *slab;
   uint64_t slab_bytes;                   // per warp
@@ -190,6 +196,7 @@ struct EnumPlan {
   uint32_t blocks = 0, threads = 0;
   size_t smem = 0;
   uint64_t nwarps = 0, nwork = 0;
+  bool vertex_pass = false;  // a range: vertices first, then the roots they leave
   bool fits_all = false;  // every root fits the normal slab: no deferred pass possible
   uint32_t pool_blocks = 0;
   uint32_t heavy_warps = 0;  // cap on the large-scratch pass (0 = as memory allows)

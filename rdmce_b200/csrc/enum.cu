@@ -78,6 +78,9 @@ constexpr uint32_t kLocalRec = 2048;      // per-warp local task record (64-bit-
 // with fewer, larger tasks, once nested tiers expose their outer levels first.
 constexpr uint32_t kRegShareBound = 24;
 constexpr uint32_t kShareMin = 128, kShareMax = 8192;
+// Vertex pass: the first claims (the core's vertices) take one vertex, later
+// ones kVertexChunk, since a claim costs as much as a small vertex's work.
+constexpr uint32_t kVertexChunk = 8, kVertexSingles = 8;  // single claims: kVertexSingles a warp
 // 32-bit-tier nodes with this few candidates (5, 6 or 7) are decided in one
 // step.  Larger limits take more nodes off the search tree but grow the node
 // loop's code (the instruction cache bounds the kernel): 6 measured as fast
@@ -1539,7 +1542,7 @@ __device__ bool gen_materialize(const Ctx &c, const Gen &G, const uint64_t *rec_
     h->pc = pc;
     h->nrows = nrows;
     h->W = Wn;
-    h->rsize = ((uint32_t)(m1 >> 32) & 0x7fffffffu) + 1;
+    h->rsize = ((uint32_t)(m1 >> 32) + 1) & 0x7fffffffu;
     h->s1 = rec_l[3 * W + 2] + G.h1s[q];
     h->s2 = rec_l[3 * W + 3] + G.h2s[q];
     h->slot = c.sm->slot;
@@ -1619,7 +1622,7 @@ __device__ __noinline__ void gen_solve_body(Ctx c, Gen G, uint32_t rsize0, uint6
   if (lane == 0) {
     uint64_t *m = stack + 3 * W;
     m[0] = (uint64_t)kIdent | ((uint64_t)G.nrows << 32);
-    m[1] = (uint64_t)rsize0 << 32;
+    m[1] = (uint64_t)(rsize0 & 0x7fffffffu) << 32;  // a root vertex starts at -1
     m[2] = s10;
     m[3] = s20;
   }
@@ -1658,7 +1661,7 @@ __device__ __noinline__ void gen_solve_body(Ctx c, Gen G, uint32_t rsize0, uint6
           }
           blocked = hit;
         }
-        if (!blocked && lane == 0) emit(c, rsize + 2, rec[3 * W + 2], rec[3 * W + 3]);
+        if (!blocked && lane == 0) emit(c, (rsize + 2) & 0x7fffffffu, rec[3 * W + 2], rec[3 * W + 3]);
         fresh = false;
         if (level == 0) break;
         level--;
@@ -1855,7 +1858,7 @@ __device__ __noinline__ void gen_solve_body(Ctx c, Gen G, uint32_t rsize0, uint6
     }
     if (lane == 0) {
       crec[3 * W] = (uint64_t)caoff | ((uint64_t)calen << 32);
-      crec[3 * W + 1] = (uint64_t)catop | ((uint64_t)rs << 32) | (clazy ? (1ULL << 63) : 0);
+      crec[3 * W + 1] = (uint64_t)catop | ((uint64_t)(rs & 0x7fffffffu) << 32) | (clazy ? (1ULL << 63) : 0);
       crec[3 * W + 2] = t1;
       crec[3 * W + 3] = t2;
     }
@@ -2199,6 +2202,58 @@ __device__ uint32_t build_rows_wide(const DevGraph &g, const uint32_t *cand, uin
   return nrows;
 }
 
+// Solve an ego network whose rows are in the slab, in the smallest tier that
+// holds it.  colv: the candidates' vertex ids; rsize: |R| beyond two vertices.
+__device__ __noinline__ void solve_ego(Ctx c, const uint32_t *colv, uint32_t nrows, uint32_t p, uint32_t W,
+                                       const Layout &L, uint32_t rsize, uint64_t s1, uint64_t s2) {
+  const DevGraph &g = c.P->g;
+  const uint64_t *rows = (const uint64_t *)(c.slab + L.rows_off);
+  if (p <= 32 && nrows <= 32) {
+    T0 t0;
+    t0.row = c.lane < nrows ? (uint32_t)rows[c.lane] : 0;
+    t0.cv = c.lane < p ? colv[c.lane] : 0;
+    t0.h1 = c.lane < p ? g.h1[t0.cv] : 0;
+    t0.h2 = c.lane < p ? g.h2[t0.cv] : 0;
+    __syncwarp();
+    t0_solve(c, t0, p, nrows, rsize, s1, s2);
+    return;
+  }
+  if (W == 1 && nrows <= kT1Rows) {
+    T1 t;
+#pragma unroll
+    for (int j = 0; j < kRPL; j++) {
+      const uint32_t idx = 32 * j + c.lane;
+      t.r[j] = idx < nrows ? rows[idx] : 0;
+    }
+    t.cva = c.lane < p ? colv[c.lane] : 0;
+    t.cvb = c.lane + 32 < p ? colv[c.lane + 32] : 0;
+    t1_hashes(c, t, p);
+    __syncwarp();
+    t1_solve(c, t, p, nrows, rsize, s1, s2);
+    return;
+  }
+  Gen G;
+  G.rows = rows;
+  G.colv = colv;
+  uint64_t *h1s = (uint64_t *)(c.slab + L.hash_off);
+  uint64_t *h2s = h1s + p;
+  for (uint32_t j = c.lane; j < p; j += 32) {
+    const uint32_t y = colv[j];
+    h1s[j] = g.h1[y];
+    h2s[j] = g.h2[y];
+  }
+  G.h1s = h1s;
+  G.h2s = h2s;
+  G.stack = (uint64_t *)(c.slab + L.stack_off);
+  G.alist = (uint32_t *)(c.slab + L.alist_off);
+  G.alist_cap = (c.slab_bytes - kTail - L.alist_off) / 4;
+  G.pc = p;
+  G.nrows = nrows;
+  G.W = W;
+  __syncwarp();
+  gen_solve(c, G, rsize, s1, s2);
+}
+
 // Solve root r.  Returns false when the root does not fit this slab.
 __device__ bool solve_root(const Ctx &c, uint64_t r) {
   const DevGraph &g = c.P->g;
@@ -2241,51 +2296,65 @@ __device__ bool solve_root(const Ctx &c, uint64_t r) {
   const uint32_t nrows = W <= 64 ? build_rows(g, cand, x, p, W, rows, c.sm) : build_rows_wide(g, cand, x, p, W, rows);
   __syncwarp();
   if (c.lane == 0) c.sm->cyc[kCycBuild] += now() - tb0;
-  if (p <= 32 && nrows <= 32) {
-    T0 t0;
-    t0.row = c.lane < nrows ? (uint32_t)rows[c.lane] : 0;
-    t0.cv = c.lane < p ? cand[x + c.lane] : 0;
-    t0.h1 = c.lane < p ? g.h1[t0.cv] : 0;
-    t0.h2 = c.lane < p ? g.h2[t0.cv] : 0;
-    __syncwarp();
-    t0_solve(c, t0, p, nrows, 0, s1, s2);
-    return true;
-  }
-  if (W == 1 && nrows <= kT1Rows) {
-    T1 t;
-#pragma unroll
-    for (int j = 0; j < kRPL; j++) {
-      const uint32_t idx = 32 * j + c.lane;
-      t.r[j] = idx < nrows ? rows[idx] : 0;
-    }
-    t.cva = c.lane < p ? cand[x + c.lane] : 0;
-    t.cvb = c.lane + 32 < p ? cand[x + c.lane + 32] : 0;
-    t1_hashes(c, t, p);
-    __syncwarp();
-    t1_solve(c, t, p, nrows, 0, s1, s2);
-    return true;
-  }
-  Gen G;
-  G.rows = rows;
-  G.colv = cand + x;
-  uint64_t *h1s = (uint64_t *)(c.slab + L.hash_off);
-  uint64_t *h2s = h1s + p;
-  for (uint32_t j = c.lane; j < p; j += 32) {
-    const uint32_t y = cand[x + j];
-    h1s[j] = g.h1[y];
-    h2s[j] = g.h2[y];
-  }
-  G.h1s = h1s;
-  G.h2s = h2s;
-  G.stack = (uint64_t *)(c.slab + L.stack_off);
-  G.alist = (uint32_t *)(c.slab + L.alist_off);
-  G.alist_cap = (c.slab_bytes - kTail - L.alist_off) / 4;
-  G.pc = p;
-  G.nrows = nrows;
-  G.W = W;
-  __syncwarp();
-  gen_solve(c, G, 0, s1, s2);
+  solve_ego(c, cand + x, nrows, p, W, L, 0, s1, s2);
   return true;
+}
+
+// Vertices solved whole.  Up to kVertexCols later neighbours and kVertexDegree
+// neighbours a vertex's ego network is built once and searched with a pivot;
+// from 65 later neighbours on (the general tier) only where at most
+// kVertexBranches of them, and at most a quarter, are left to branch on.
+constexpr uint32_t kVertexCols = 256, kVertexDegree = 16384, kVertexBranches = 16;
+
+// Vertex item k of the vertex pass: the cliques whose first vertex (in the
+// order) is v.  An edge root (v, w) builds its own ego network out of the
+// members' lists, so a member's list is read once for every w it is adjacent
+// to; here it is read once for v, and no intersection is needed, since v's
+// own list is the ego network's vertex set.  The pivot also skips every w that
+// it is adjacent to.  A vertex with many candidates and no good pivot is left
+// to the edge pass: its roots are many warps' work.  Returns its solved roots.
+// Measured (B200): planted cliques of 40-200 vertices in 10^5 202 -> 8.6 ms,
+// Chung-Lu 10^6 15.4 -> 9.7 ms; the root build's share of full R-MAT 14 15 % -> 1 %.
+__device__ __noinline__ uint32_t run_vertex(Ctx c, uint64_t k) {
+  const EnumParams &P = *c.P;
+  const DevGraph &g = P.g;
+  const uint32_t v = g.n - 1 - (uint32_t)k;  // late-peeled vertices first
+  const uint32_t r0 = g.root_off[v], r1 = g.root_off[v + 1];
+  const uint32_t lo = (uint32_t)max((uint64_t)r0, P.rb), hi = (uint32_t)min((uint64_t)r1, P.re);
+  if (lo >= hi) return 0;
+  const unsigned long long t0 = now();
+  const uint32_t b = g.off[v], d = g.off[v + 1] - b, p = r1 - r0, x = d - p, W = (p + 63) / 64;
+  const Layout L = layout_for(0, p, d, W);
+  bool whole = hi - lo == p && p <= kVertexCols && d <= kVertexDegree && L.need <= c.slab_bytes;
+  if (whole) {
+    const uint32_t *cand = g.adj + b;
+    uint64_t *rows = (uint64_t *)(c.slab + L.rows_off);
+    set_slot(c, g.slot ? g.slot[v] : 0);
+    const uint32_t nrows = build_rows(g, cand, x, p, W, rows, c.sm);
+    __syncwarp();
+    if (W > 1) {
+      uint32_t best = p;
+      for (uint32_t r = c.lane; r < nrows; r += 32) {
+        uint32_t n = 0;
+        for (uint32_t w = 0; w < W; w++) n += __popcll(rows[(uint64_t)r * W + w]);
+        best = min(best, p - n);
+      }
+      best = __reduce_min_sync(kFull, best);
+      whole = best <= kVertexBranches && 4 * best <= p;
+    }
+    if (c.lane == 0) c.sm->cyc[kCycBuild] += now() - t0;
+    // |R| is counted beyond a root edge: one less for a root vertex
+    if (whole) solve_ego(c, cand + x, nrows, p, W, L, 0xffffffffu, g.h1[v], g.h2[v]);
+  }
+  if (!whole) {
+    uint32_t at = 0;
+    if (c.lane == 0) at = atomicAdd(P.edge_n, hi - lo);
+    at = __shfl_sync(kFull, at, 0);
+    for (uint32_t i = c.lane; i < hi - lo; i += 32) P.edge_out[at + i] = hi - 1 - i;
+  }
+  if (c.lane == 0) atomicMax(P.stat_max_item, now() - t0);
+  __syncwarp();
+  return whole ? p : 0;
 }
 
 // Solve a task popped from the pool; the block goes back to the free ring as
@@ -2357,7 +2426,7 @@ __device__ __noinline__ void run_root(Ctx c, uint64_t k) {
   // wk: the root's index in this solve's work list (per-root results are
   // kept by it); the large-scratch pass walks a list of such indices
   const uint64_t wk = P.heavy_list ? P.heavy_list[k] : k;
-  const uint64_t r = P.root_list ? P.root_list[wk] : P.re - 1 - wk;  // range: late-peeled roots first
+  const uint64_t r = P.edge_list ? P.edge_list[wk] : P.root_list ? P.root_list[wk] : P.re - 1 - wk;  // range: late-peeled roots first
   const unsigned long long c0 = sm->count, h0 = sm->checksum;
   const unsigned long long tr = now();
   const bool fit = solve_root(c, r);
@@ -2488,7 +2557,11 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
   c.slab_bytes = P.slab_bytes;
   c.ta = (T1Area *)(c.slab + c.slab_bytes - kTail);
   c.sharing = P.sharing != 0;
-  const uint64_t total = P.heavy_list ? P.n_heavy : (P.root_list ? P.n_list : P.re - P.rb);
+  const uint64_t total = P.heavy_list    ? P.n_heavy
+                         : P.vertex_pass ? P.single_items + (P.g.n - P.single_items + kVertexChunk - 1) / kVertexChunk
+                         : P.edge_list   ? *P.edge_n
+                         : P.root_list   ? P.n_list
+                                         : P.re - P.rb;
   unsigned long long nroots = 0;
   // a warp counts itself busy from its first root claim until a claim fails,
   // so warps that start late (not co-resident) are never waited for
@@ -2515,6 +2588,15 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
     if (c.lane == 0) k = atomicAdd(P.next, 1ULL);
     k = __shfl_sync(kFull, k, 0);
     if (k >= total) break;
+    if (P.vertex_pass) {
+      uint64_t v = k, e = k + 1;
+      if (k >= P.single_items) {
+        v = P.single_items + (k - P.single_items) * kVertexChunk;
+        e = min(v + kVertexChunk, (uint64_t)P.g.n);
+      }
+      for (; v < e; v++) nroots += run_vertex(c, v);
+      continue;
+    }
     nroots++;
     run_root(c, k);
   }
@@ -2548,6 +2630,7 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
 // Control words; the contended ones each own a 128-byte line.
 struct EnumCtl {
   alignas(128) unsigned long long next;
+  alignas(128) unsigned long long next_edge;  // claims of the edge pass
   alignas(128) unsigned long long free_head;
   alignas(128) unsigned long long free_tail;
   alignas(128) unsigned long long ready_head;
@@ -2556,7 +2639,7 @@ struct EnumCtl {
   alignas(128) unsigned long long heavy_need, stat_roots, stat_tasks, stat_nodes, stat_wops, stat_bbytes;
   unsigned long long stat_cycles[kCycPhases];
   unsigned long long stat_max_item[2];
-  unsigned int heavy_n, error;
+  unsigned int heavy_n, error, edge_n;
 };
 
 // free ring full of every block, ready ring empty, counters reset
@@ -2584,6 +2667,15 @@ mce_status reset_ctl(const EnumPlan &plan, cudaStream_t st) {
   return MCE_OK;
 }
 
+// the launch behind the vertex pass: the roots that pass left
+EnumParams edge_pass(const EnumPlan &plan) {
+  EnumParams P = plan.params;
+  P.vertex_pass = 0;
+  P.edge_list = P.edge_out;
+  P.next = &((EnumCtl *)plan.ctl)->next_edge;
+  return P;
+}
+
 }  // namespace
 
 mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, Scratch *scr, SlotResult *slots,
@@ -2604,6 +2696,7 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   P.g.h2 = g.h2;
   P.g.root_v0 = g.root_v0;
   P.g.root_v1 = g.root_v1;
+  P.g.root_off = g.root_off;
   P.g.slot = g.slot;
   P.slots = slots;
   P.hist = hist;
@@ -2698,6 +2791,16 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   P.re = re;
   P.root_list = list_mode ? cfg.root_list : nullptr;
   P.n_list = list_mode ? cfg.n_root_list : 0;
+  // A range goes vertex by vertex first; per-root values and the counters of
+  // the edge-rooted method (stats) need every root on its own.
+  plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && nwork;
+  if (plan->vertex_pass) {
+    P.edge_out = (uint32_t *)scr->get(8, nwork * 4, &s);
+    if (!P.edge_out) return s;
+    P.edge_n = &ctl->edge_n;
+    P.vertex_pass = 1;
+    P.single_items = std::min<uint64_t>(g.n, kVertexSingles * nwarps);
+  }
   P.heavy_out = heavy;
   P.heavy_cap = (uint32_t)heavy_cap;
   P.push_heavy = 1;
@@ -2718,6 +2821,10 @@ mce_status MCE_ENUM_FN(enum_launch)(const EnumPlan &plan, cudaStream_t st) {
   if (plan.nwork) {
     k_enumerate<<<plan.blocks, plan.threads, plan.smem, st>>>(plan.params);
     note_launch();
+    if (plan.vertex_pass) {
+      k_enumerate<<<plan.blocks, plan.threads, plan.smem, st>>>(edge_pass(plan));
+      note_launch();
+    }
     MCE_CUDA_TRY(cudaGetLastError());
   }
   return MCE_OK;
@@ -2729,7 +2836,7 @@ mce_status MCE_ENUM_FN(enum_finish)(const EnumPlan &plan, cudaStream_t st, EnumS
   MCE_CUDA_TRY(cudaMemcpyAsync(&h, ctl, sizeof(EnumCtl), cudaMemcpyDeviceToHost, st));
   MCE_CUDA_TRY(cudaStreamSynchronize(st));
   const uint64_t heavy_roots = h.heavy_n;
-  uint64_t launches = plan.nwork ? 1 : 0;
+  uint64_t launches = plan.nwork ? (plan.vertex_pass ? 2 : 1) : 0;
   uint64_t roots = h.stat_roots;
   uint64_t tasks = h.stat_tasks, nodes = h.stat_nodes, wops = h.stat_wops, bbytes = h.stat_bbytes;
   uint64_t cycles[kCycPhases];
@@ -2750,6 +2857,8 @@ mce_status MCE_ENUM_FN(enum_finish)(const EnumPlan &plan, cudaStream_t st, EnumS
     hw = std::min<uint64_t>(hw, h.heavy_n);
     if (hw == 0) return MCE_ERR_OUT_OF_MEMORY;
     EnumPlan H = plan;
+    if (H.vertex_pass) H.params = edge_pass(plan);  // the list holds indices of that pass
+    H.params.next = &ctl->next;
     const uint32_t wpb = plan.threads / 32;
     if (hw < wpb) {
       H.blocks = 1;

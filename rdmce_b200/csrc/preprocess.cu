@@ -275,6 +275,12 @@ __global__ void k_roots(const uint64_t *keys, uint64_t m2, int nb, const uint32_
     }
 }
 
+// first root of each vertex: the roots before its row
+__global__ void k_root_off(const uint32_t *off, const uint32_t *pos, uint32_t n, uint32_t *root_off) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x)
+    root_off[v] = pos[off[v]];
+}
+
 __global__ void k_permute_labels(const uint32_t *labels_old, const uint32_t *rank, uint32_t n, uint32_t *labels,
                                  uint64_t *h1, uint64_t *h2) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -629,6 +635,8 @@ mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32
   MCE_CUDA_TRY(cudaMallocAsync(&g->root_v0, std::max<uint64_t>(m, 1) * sizeof(uint32_t), st));
   MCE_CUDA_TRY(cudaMallocAsync(&g->root_v1, std::max<uint64_t>(m, 1) * sizeof(uint32_t), st));
   k_roots<<<grid_for(m2, 256), 256, 0, st>>>(keys.p, m2, nb, upflag.p, uppos.p, g->root_v0, g->root_v1); note_launch();
+  MCE_CUDA_TRY(cudaMallocAsync(&g->root_off, (n + 1) * sizeof(uint32_t), st));
+  k_root_off<<<grid_for(n + 1, 256), 256, 0, st>>>(g->off, uppos.p, n, g->root_off); note_launch();
   keys.release();
 
   // 5) labels and their hashes under the new ids
@@ -718,6 +726,7 @@ void free_graph(DeviceGraph *g) {
   cudaFreeAsync(g->h2, st);
   cudaFreeAsync(g->root_v0, st);
   cudaFreeAsync(g->root_v1, st);
+  cudaFreeAsync(g->root_off, st);
   if (g->slot) cudaFreeAsync(g->slot, st);
   *g = DeviceGraph{};
 }
