@@ -185,6 +185,7 @@ struct EnumParams {
   uint32_t *free_slot, *ready_slot;
   unsigned long long *free_seq, *ready_seq;
   unsigned long long *free_head, *free_tail, *ready_head, *ready_tail;
+  int *free_count, *ready_count;         // filled cells not yet claimed
 };
 
 

@@ -276,9 +276,17 @@ __device__ __forceinline__ void maybe_flush(const Ctx &c) {
 // ------------------------------------------------------- bounded MPMC rings
 // Vyukov's bounded queue: cell seq == pos means free for the producer of pos,
 // seq == pos + 1 means filled for the consumer of pos.  Lane 0 only.
+//
+// A consumer first takes one of the ring's filled cells off its count, then
+// draws its position with an unconditional add.  Advancing the head by
+// compare-and-swap instead lets one consumer through in each round trip to L2
+// while all others retry: with hundreds of idle warps polling, that capped the
+// task rate at 1.3-2.8 tasks a microsecond however many warps were idle.
+// Measured (B200): 1024 core roots of R-MAT 20 43.7 -> 27.7 ms, full R-MAT 14
+// 31.9 -> 20.9 ms.
 
-__device__ bool ring_push(uint32_t *slots, unsigned long long *seq, unsigned long long *tail, uint32_t mask,
-                          uint32_t val, const EnumParams &P) {
+__device__ bool ring_push(uint32_t *slots, unsigned long long *seq, unsigned long long *tail, int *count,
+                          uint32_t mask, uint32_t val, const EnumParams &P) {
   const unsigned long long pos = atomicAdd(tail, 1ULL);
   volatile unsigned long long *s = seq + (pos & mask);
   uint64_t n = 0;
@@ -292,33 +300,34 @@ __device__ bool ring_push(uint32_t *slots, unsigned long long *seq, unsigned lon
   ((volatile uint32_t *)slots)[pos & mask] = val;
   __threadfence();
   *s = pos + 1;
+  __threadfence();
+  atomicAdd(count, 1);
   return true;
 }
 
-__device__ bool ring_pop(uint32_t *slots, unsigned long long *seq, unsigned long long *head,
-                         unsigned long long *tail, uint32_t mask, uint32_t *val, const EnumParams &P) {
-  for (int tries = 0; tries < 8; tries++) {
-    const unsigned long long h = *(volatile unsigned long long *)head;
-    const unsigned long long t = *(volatile unsigned long long *)tail;
-    if (h >= t) return false;
-    if (atomicCAS(head, h, h + 1) == h) {
-      volatile unsigned long long *s = seq + (h & mask);
-      uint64_t n = 0;
-      while (*s != h + 1) {
-        if (++n > P.spin_limit) {
-          atomicExch(P.error, 3u);
-          return false;
-        }
-        __nanosleep(32);
-      }
-      __threadfence();
-      *val = ((volatile uint32_t *)slots)[h & mask];
-      __threadfence();
-      *s = h + (unsigned long long)mask + 1;
-      return true;
-    }
+__device__ bool ring_pop(uint32_t *slots, unsigned long long *seq, unsigned long long *head, int *count,
+                         uint32_t mask, uint32_t *val, const EnumParams &P) {
+  if (*(volatile int *)count <= 0) return false;
+  if (atomicSub(count, 1) <= 0) {  // others were quicker
+    atomicAdd(count, 1);
+    return false;
   }
-  return false;
+  const unsigned long long h = atomicAdd(head, 1ULL);
+  volatile unsigned long long *s = seq + (h & mask);
+  uint64_t n = 0;
+  // a cell counted as filled may lie behind one whose producer is still writing
+  while (*s != h + 1) {
+    if (++n > P.spin_limit) {
+      atomicExch(P.error, 3u);
+      return false;
+    }
+    __nanosleep(32);
+  }
+  __threadfence();
+  *val = ((volatile uint32_t *)slots)[h & mask];
+  __threadfence();
+  *s = h + (unsigned long long)mask + 1;
+  return true;
 }
 
 // warp-uniform wrappers
@@ -326,7 +335,7 @@ __device__ __forceinline__ bool pool_alloc(const Ctx &c, uint32_t *blk) {
   const EnumParams &P = *c.P;
   uint32_t b = 0;
   bool ok = false;
-  if (c.lane == 0) ok = ring_pop(P.free_slot, P.free_seq, P.free_head, P.free_tail, P.pool_mask, &b, P);
+  if (c.lane == 0) ok = ring_pop(P.free_slot, P.free_seq, P.free_head, P.free_count, P.pool_mask, &b, P);
   ok = __shfl_sync(kFull, ok, 0);
   *blk = __shfl_sync(kFull, b, 0);
   return ok;
@@ -335,7 +344,7 @@ __device__ __forceinline__ bool pool_alloc(const Ctx &c, uint32_t *blk) {
 __device__ __forceinline__ void pool_free(const Ctx &c, uint32_t blk) {
   const EnumParams &P = *c.P;
   __syncwarp();
-  if (c.lane == 0) ring_push(P.free_slot, P.free_seq, P.free_tail, P.pool_mask, blk, P);
+  if (c.lane == 0) ring_push(P.free_slot, P.free_seq, P.free_tail, P.free_count, P.pool_mask, blk, P);
   __syncwarp();
 }
 
@@ -345,7 +354,7 @@ __device__ __forceinline__ void pool_publish(const Ctx &c, uint32_t blk) {
   __syncwarp();
   if (c.lane == 0) {
     __threadfence();
-    ring_push(P.ready_slot, P.ready_seq, P.ready_tail, P.pool_mask, blk, P);
+    ring_push(P.ready_slot, P.ready_seq, P.ready_tail, P.ready_count, P.pool_mask, blk, P);
     atomicAdd(P.stat_tasks, 1ULL);
   }
   __syncwarp();
@@ -361,10 +370,8 @@ __device__ __forceinline__ bool hungry(const Ctx &c) {
   uint32_t h = 0;
   if (c.lane == 0) {
     const uint32_t active = *(volatile unsigned int *)P.active;
-    const unsigned long long rh = *(volatile unsigned long long *)P.ready_head;
-    const unsigned long long rt = *(volatile unsigned long long *)P.ready_tail;
-    const uint64_t queued = rt > rh ? rt - rh : 0;
-    const uint32_t idle = P.nwarps > active ? P.nwarps - active : 0;
+    const int queued = *(volatile int *)P.ready_count;
+    const int idle = (int)P.nwarps - (int)active;
     h = idle > 0 && queued < idle;
   }
   return __shfl_sync(kFull, h, 0) != 0;
@@ -2495,12 +2502,10 @@ __device__ __noinline__ int idle_wait(Ctx c, unsigned int *s_poll) {
         polled = true;
         const uint32_t act = *(volatile unsigned int *)P.active;
         __threadfence();
-        const unsigned long long rh = *(volatile unsigned long long *)P.ready_head;
-        const unsigned long long rt = *(volatile unsigned long long *)P.ready_tail;
-        if (rh < rt) {
+        if (*(volatile int *)P.ready_count > 0) {
           seen = true;
           uint32_t b = 0;
-          if (ring_pop(P.ready_slot, P.ready_seq, P.ready_head, P.ready_tail, P.pool_mask, &b, P)) {
+          if (ring_pop(P.ready_slot, P.ready_seq, P.ready_head, P.ready_count, P.pool_mask, &b, P)) {
             atomicAdd(P.active, 1u);
             result = (int)b;
           }
@@ -2573,7 +2578,7 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
       bool got = false;
       uint32_t b = 0;
       const unsigned long long tq = now();
-      if (c.lane == 0) got = ring_pop(P.ready_slot, P.ready_seq, P.ready_head, P.ready_tail, P.pool_mask, &b, P);
+      if (c.lane == 0) got = ring_pop(P.ready_slot, P.ready_seq, P.ready_head, P.ready_count, P.pool_mask, &b, P);
       got = __shfl_sync(kFull, got, 0);
       const uint32_t blk = __shfl_sync(kFull, b, 0);
       if (c.lane == 0) sm->cyc[kCycQueue] += now() - tq;
@@ -2635,6 +2640,8 @@ struct EnumCtl {
   alignas(128) unsigned long long free_tail;
   alignas(128) unsigned long long ready_head;
   alignas(128) unsigned long long ready_tail;
+  alignas(128) int ready_count;  // filled cells not yet claimed
+  alignas(128) int free_count;
   alignas(128) unsigned int active;
   alignas(128) unsigned long long heavy_need, stat_roots, stat_tasks, stat_nodes, stat_wops, stat_bbytes;
   unsigned long long stat_cycles[kCycPhases];
@@ -2654,7 +2661,10 @@ __global__ void k_pool_init(EnumCtl *ctl, uint32_t *free_slot, unsigned long lon
   if (blockIdx.x == 0) {
     for (uint32_t w = threadIdx.x; w < sizeof(EnumCtl) / 4; w += blockDim.x) ((uint32_t *)ctl)[w] = 0;
     __syncthreads();
-    if (threadIdx.x == 0) ctl->free_tail = n;
+    if (threadIdx.x == 0) {
+      ctl->free_tail = n;
+      ctl->free_count = (int)n;
+    }
   }
 }
 
@@ -2729,6 +2739,8 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   P.free_tail = &ctl->free_tail;
   P.ready_head = &ctl->ready_head;
   P.ready_tail = &ctl->ready_tail;
+  P.ready_count = &ctl->ready_count;
+  P.free_count = &ctl->free_count;
 
   uint64_t rb = cfg.root_begin, re = cfg.root_end ? std::min<uint64_t>(cfg.root_end, g.m) : g.m;
   if (rb > re) rb = re;
