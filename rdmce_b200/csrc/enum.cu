@@ -81,16 +81,13 @@ constexpr uint32_t kShareMin = 128, kShareMax = 8192;
 // Vertex pass: the first claims (the core's vertices) take one vertex, later
 // ones kVertexChunk, since a claim costs as much as a small vertex's work.
 constexpr uint32_t kVertexChunk = 8, kVertexSingles = 8;  // single claims: kVertexSingles a warp
-// 32-bit-tier nodes with this few candidates (5, 6 or 7) are decided in one
-// step.  Larger limits take more nodes off the search tree but grow the node
-// loop's code (the instruction cache bounds the kernel): 6 measured as fast
-// as 5 where the join decision below takes most nodes, and 7 % faster where
-// it does not (active rows outside P); 7 was slower.
+// 32-bit-tier nodes with up to this many candidates are decided in one step,
+// at 2^(n - 5) groups of about 12 instructions each (t0_small_sets).
 #ifndef MCE_SMALL_P
-#define MCE_SMALL_P 6
+#define MCE_SMALL_P 9
 #endif
 constexpr int kSmallP = MCE_SMALL_P;
-static_assert(kSmallP >= 5 && kSmallP <= 7, "small-node decisions cover up to 5, 6 or 7 candidates");
+static_assert(kSmallP >= 5 && kSmallP <= 12, "small-node decisions: groups double with each candidate");
 // phases of the per-warp cycle accounting
 // (kCycReg: the 64-bit tier; kCycT0: the 32-bit tier)
 enum { kCycBuild = 0, kCycReg = 1, kCycGen = 2, kCycSpawn = 3, kCycIdle = 4, kCycQueue = 5, kCycT0 = 6, kCycPhases = 7 };
@@ -112,6 +109,13 @@ __host__ __device__ __forceinline__ uint64_t align8(uint64_t x) { return (x + 7)
 __host__ __device__ __forceinline__ uint64_t task_bytes(uint32_t pc, uint32_t nrows, uint32_t W) {
   return kHdr + align8(4ULL * pc) + 8ULL * nrows * W;
 }
+
+// A compression plan (compress_plan): the selected bits and the six move masks.
+struct CPlan {
+  uint64_t m;
+  uint64_t mv[6];
+};
+static_assert(sizeof(CPlan) == 56, "layout_for reserves this much a word");
 
 // A general-tier subproblem laid out in the warp's slab.
 struct Gen {
@@ -140,9 +144,14 @@ struct WarpSmem {
   uint64_t t0_s1, t0_s2;
   uint32_t t0_rsize;
   uint32_t pend_rm[32];
+  // collected small nodes (t0_batch): candidate k's row of node i at
+  // [33 k + i] (a row stride of 33 keeps one node's rows in different banks),
+  // the candidates and R
+  uint32_t pr_row[33 * kSmallP];
+  uint32_t pr_P[32], pr_RM[32];
   uint64_t lchk[32];  // per-lane checksum accumulators (batched leaves)
   // a 32-bit-tier solve that stepped out to expose work: its node state
-  uint32_t y_P, y_A, y_RM, y_npend;
+  uint32_t y_P, y_A, y_RM, y_npend, y_nprob;
   int y_level;
   // nodes between the 32-bit tier's checks for idle warps; doubles (up to
   // kShareMax) while checks find nothing to expose, back to kShareMin after
@@ -382,11 +391,6 @@ __device__ __forceinline__ bool hungry(const Ctx &c) {
 // end (Hacker's Delight 2nd ed. section 7-4, parallel-suffix form).  The plan
 // depends only on m, which is warp-uniform wherever it is used.
 
-struct CPlan {
-  uint64_t m;
-  uint64_t mv[6];
-};
-
 __device__ __forceinline__ CPlan compress_plan(uint64_t m) {
   CPlan p;
   p.m = m;
@@ -461,20 +465,16 @@ struct T0 {
   uint64_t h1, h2;  // label hashes of column lane
 };
 
-// Hash the pending leaves, one per lane: sums of the entry sums and the R
+// Hash one leaf per live lane (R = rm): sums of the entry sums and the R
 // columns' hashes, then the clique hash, histogram and largest size.
 // Out of line: it runs once per 32 leaves, and one copy keeps the hot node
 // loop's code small (instruction-cache misses, not issue slots, bound it).
-__device__ __noinline__ void t0_flush(Ctx c, uint32_t npend, uint64_t s10, uint64_t s20,
-                                         uint32_t rsize0) {
-  WarpSmem *sm = c.sm;
-  const uint32_t lane = c.lane;
-  __syncwarp();
+__device__ __noinline__ void t0_hash(const EnumParams *Pm, WarpSmem *sm, uint32_t rm, bool live) {
+  const uint32_t lane = lane_id();
   uint32_t size = 0;
-  if (lane < npend) {
-    uint32_t rm = sm->pend_rm[lane];
-    size = rsize0 + 2 + __popc(rm);
-    uint64_t a = s10, b = s20;
+  if (live) {
+    size = sm->t0_rsize + 2 + __popc(rm);
+    uint64_t a = sm->t0_s1, b = sm->t0_s2;
     while (rm) {
       const uint32_t i = __ffs(rm) - 1;
       rm &= rm - 1;
@@ -485,18 +485,25 @@ __device__ __noinline__ void t0_flush(Ctx c, uint32_t npend, uint64_t s10, uint6
     if (size < kHistCache) {
       atomicAdd(&sm->hcache[size], 1u);
     } else {
-      const EnumParams &P = *c.P;
-      const uint32_t bin = size < P.hist_len ? size : P.hist_len - 1;
-      atomicAdd(&P.hist[(uint64_t)sm->slot * P.hist_len + bin], 1ULL);
+      const uint32_t bin = size < Pm->hist_len ? size : Pm->hist_len - 1;
+      atomicAdd(&Pm->hist[(uint64_t)sm->slot * Pm->hist_len + bin], 1ULL);
     }
   }
+  const uint32_t n = __popc(__ballot_sync(kFull, live));
   const uint32_t mx = __reduce_max_sync(kFull, size);
   if (lane == 0) {
-    sm->count += npend;
-    sm->pending += npend;
+    sm->count += n;
+    sm->pending += n;
     sm->max_size = max(sm->max_size, mx);
   }
   __syncwarp();
+}
+
+// hash the pending leaves
+__device__ __forceinline__ void t0_flush(const Ctx &c, uint32_t npend) {
+  __syncwarp();
+  const bool live = c.lane < npend;
+  t0_hash(c.P, c.sm, live ? c.sm->pend_rm[c.lane] : 0u, live);
 }
 
 // hash sums of a frame's R mask (lanes of R contribute their column hash)
@@ -574,147 +581,177 @@ __device__ bool t0_spawn(const Ctx &c, const T0 &t, int level) {
   return true;
 }
 
-// Lanes whose index has bit k set: lane s stands for the subset s of a small
-// node's candidates (bit k = its k-th lowest candidate).
-__device__ __forceinline__ constexpr uint32_t lanes_with_bit(int k) {
-  return k == 0 ? 0xAAAAAAAAu : k == 1 ? 0xCCCCCCCCu : k == 2 ? 0xF0F0F0F0u : k == 3 ? 0xFF00FF00u : 0xFFFF0000u;
-}
-
-// A node with exactly N (3..7) candidates, decided in one step.  R + K is a
-// maximal clique for exactly the cliques K of the candidates that no active
-// row contains (a candidate outside K that extends K is itself such a row).
-// The subsets are numbered s = 32 g + lane: the lane index carries the
-// subset's lowest five candidates, the group g (one pass each, 2^(N-5) of
-// them) the rest.  Whether s is a clique is read off warp-uniform masks: a
-// missing edge (i, j) among the lane's candidates excludes the lanes with bits
-// i and j; a missing edge from a group candidate u to candidate i excludes the
-// lanes with bit i in the groups holding u; a missing edge between two group
-// candidates excludes whole groups.  Rows containing s: the AND of the
-// per-candidate ballots over s's members.
-template <int N>
-__device__ __forceinline__ void t0_small_n(const Ctx &c, const T0 &t, uint32_t P, uint32_t A, uint32_t RM,
-                                           uint32_t &npend, uint64_t s10, uint64_t s20, uint32_t rsize0) {
-  constexpr int NL = N < 5 ? N : 5;  // candidates carried by the lane index
-  constexpr int NG = N - NL;         // candidates carried by the group
+// A node with 2 to kSmallP candidates P, active rows A and R = RM, decided in
+// one step.  R + K is a maximal clique for exactly the cliques K of the
+// candidates that no active row contains (a candidate outside K that extends K
+// is itself such a row).  A subset is a lane number b (bit k: the k-th lowest
+// candidate, for the low five) and a set of the others (a group); the subsets
+// of one group are one 32-bit word.  Every lane marks the subsets that its row
+// rules out: those the row contains and, if the row is a candidate, those that
+// hold it and a candidate it is not adjacent to.  Inside a group both depend
+// only on whether the row holds the group's members, so a lane has its two
+// words ready, and a group costs a select, one redux over the warp and the
+// leaves of what is left, which every lane knows; lane b writes subset b's.
+// A search tree spends about 250 instructions on a node and its share of
+// leaves; a group takes about 12.
+__device__ __forceinline__ void t0_small_sets(const Ctx &c, uint32_t row, uint32_t P, uint32_t A, uint32_t RM,
+                                              uint32_t &npend) {
   WarpSmem *sm = c.sm;
-  const uint32_t lane = c.lane;
-  uint32_t qb[N], h[N], r[N - 1];
-  uint32_t pm = P;
+  const uint32_t lane = c.lane, lanebit = 1u << lane;
+  uint32_t sub = 1;   // subsets of the low candidates that the row contains
+  uint32_t mask = RM; // R and this lane's subset of the low candidates
+  uint32_t high = P;
 #pragma unroll
-  for (int k = 0; k < N; k++) {
-    qb[k] = pm & (0u - pm);
-    pm ^= qb[k];
+  for (int k = 0; k < 5; k++) {  // past the last candidate: qb = 0, nothing happens
+    const uint32_t qb = high & (0u - high);
+    high ^= qb;
+    if (row & qb) sub |= sub << (1 << k);
+    if ((lane >> k) & 1) mask |= qb;
   }
-  // independent collectives: rows holding each candidate, the candidates' rows
-#pragma unroll
-  for (int k = 0; k < N; k++) h[k] = A & __ballot_sync(kFull, (t.row & qb[k]) != 0);
-#pragma unroll
-  for (int k = 0; k < N - 1; k++) r[k] = __shfl_sync(kFull, t.row, __ffs(qb[k]) - 1);
-  uint32_t notclique = 0;
-#pragma unroll
-  for (int i = 0; i < NL - 1; i++)
-#pragma unroll
-    for (int j = i + 1; j < NL; j++)
-      if (!(r[i] & qb[j])) notclique |= lanes_with_bit(i) & lanes_with_bit(j);
-  uint32_t rows = A, mask = RM;
-#pragma unroll
-  for (int k = 0; k < NL; k++)
-    if ((lane >> k) & 1) {
-      rows &= h[k];
-      mask |= qb[k];
-    }
-  const bool lane_ok = lane < (1u << NL) && !((notclique >> lane) & 1);
-#pragma unroll
-  for (int g = 0; g < (1 << NG); g++) {
-    bool ok = lane_ok && (g != 0 || lane != 0);
-    bool group_clique = true;
-    uint32_t rg = rows, mg = mask;
-#pragma unroll
-    for (int b = 0; b < NG; b++) {
-      if (!((g >> b) & 1)) continue;
-      const int u = NL + b;
-      uint32_t far = 0;  // lanes holding a candidate not adjacent to u
-#pragma unroll
-      for (int i = 0; i < NL; i++)
-        if (!(r[i] & qb[u])) far |= lanes_with_bit(i);
-      ok = ok && !((far >> lane) & 1);
-      rg &= h[u];
-      mg |= qb[u];
-#pragma unroll
-      for (int b2 = b + 1; b2 < NG; b2++)
-        if (((g >> b2) & 1) && !(r[u] & qb[NL + b2])) group_clique = false;
-    }
-    const bool out = group_clique && ok && rg == 0;
-    const uint32_t E = __ballot_sync(kFull, out);
-    const uint32_t pos = npend + __popc(E & lanemask_lt());
-    if (out && pos < 32) sm->pend_rm[pos] = mg;
-    npend += __popc(E);
-    if (npend >= 32) {
-      t0_flush(c, 32, s10, s20, rsize0);
-      if (out && pos >= 32) sm->pend_rm[pos - 32] = mg;
-      npend -= 32;
-    }
+  const bool active = A & lanebit, mine = high & lanebit;
+  // subsets ruled out where the row holds the group's (other) members, and where not
+  uint32_t dead_in = active ? sub : 0, dead_out = 0;
+  const uint32_t low = P ^ high;
+  if (low & lanebit) {  // candidate i of the low five: subsets with i need the row to hold the rest
+    const uint32_t i = __popc(low & lanemask_lt());
+    const uint32_t with_i = i == 0   ? 0xAAAAAAAAu
+                            : i == 1 ? 0xCCCCCCCCu
+                            : i == 2 ? 0xF0F0F0F0u
+                            : i == 3 ? 0xFF00FF00u
+                                     : 0xFFFF0000u;
+    dead_in |= with_i & ~(sub << (1u << i));
+    dead_out = with_i;
   }
-}
-
-// A node with 1 to kSmallP candidates P, active rows A and R = RM, decided
-// in one step: its maximal cliques go to the pending leaves.
-__device__ __forceinline__ void t0_small(const Ctx &c, const T0 &t, uint32_t P, uint32_t A, uint32_t RM,
-                                         uint32_t &npend, uint64_t s10, uint64_t s20, uint32_t rsize0) {
-  WarpSmem *sm = c.sm;
-  const uint32_t lane = c.lane;
-  if ((P & (P - 1)) == 0) {
-    // One candidate q: R + q is maximal iff no active row holds q (the pivot
-    // step would prune on such a row, else branch on q into a leaf).
-    if ((A & __ballot_sync(kFull, (t.row & P) != 0)) == 0) {
-      if (lane == 0) sm->pend_rm[npend] = RM | P;
-      if (++npend == 32) {
-        t0_flush(c, 32, s10, s20, rsize0);
-        npend = 0;
+  const uint32_t miss = high & ~row & ~lanebit;  // members the row does not hold
+  const uint32_t n = __popc(P);
+  const uint32_t all = n >= 5 ? 0xffffffffu : (1u << (1u << n)) - 1;
+  uint32_t members = 0;
+#pragma unroll 1
+  do {
+    const bool out_row = members & miss;
+    uint32_t dead = out_row ? dead_out : dead_in;
+    if (mine && (members & lanebit)) dead = out_row ? 0xffffffffu : ~sub;
+    const uint32_t E = all & ~__reduce_or_sync(kFull, dead);
+    if (E) {
+      const bool out = E & lanebit;
+      const uint32_t pos = npend + __popc(E & lanemask_lt());
+      const uint32_t leaf = mask | members;
+      if (out && pos < 32) sm->pend_rm[pos] = leaf;
+      npend += __popc(E);
+      if (npend >= 32) {
+        t0_flush(c, 32);
+        if (out && pos >= 32) sm->pend_rm[pos - 32] = leaf;
+        npend -= 32;
       }
     }
-    return;
+    members = (members - high) & high;  // the next set of high candidates, back to none after the last
+  } while (members);
+}
+
+// The leaf of an entry of t0_batch: its fixed columns and the low candidates
+// its subset number selects.
+__device__ __forceinline__ uint32_t batch_leaf(const WarpSmem *sm, uint32_t fixed, uint32_t entry) {
+  uint32_t P = sm->pr_P[entry >> 5], leaf = fixed;
+#pragma unroll
+  for (int k = 0; k < 5; k++) {
+    const uint32_t qb = P & (0u - P);
+    P ^= qb;
+    if ((entry >> k) & 1) leaf |= qb;
   }
-  {
-    const uint32_t lo = P & (0u - P), hi = P & ~lo;
-    if (hi == (hi & (0u - hi))) {
-      // Two candidates a, b.  Adjacent: R + a + b is the only maximal clique
-      // below, iff no active row holds both.  Not adjacent: R + a and R + b
-      // each are, iff no active row holds that vertex.  (What the pivot and
-      // the two branches would find.)
-      const uint32_t ra = A & __ballot_sync(kFull, (t.row & lo) != 0);
-      const uint32_t rb = A & __ballot_sync(kFull, (t.row & hi) != 0);
-      const uint32_t a = __ffs(lo) - 1;
-      uint32_t emit_rm[2];
-      uint32_t ne = 0;
-      if (__shfl_sync(kFull, t.row, a) & hi) {
-        if ((ra & rb) == 0) emit_rm[ne++] = RM | P;
-      } else {
-        if (ra == 0) emit_rm[ne++] = RM | lo;
-        if (rb == 0) emit_rm[ne++] = RM | hi;
+  return leaf;
+}
+
+// Collected small nodes without X rows, one node per lane: the same subset
+// words as t0_small_sets, with the candidates' rows taken in turn instead of
+// one per lane, so 32 nodes cost what 3 to 5 cost there.  Leaves are queued
+// and hashed 32 at a time.
+// Measured (B200): full R-MAT 15 (edge factor 16; 5.4e9 cliques, nine small
+// nodes in ten have no X rows) 482 -> 391 ms against deciding each by itself
+// (t0_small_sets), 562 ms with one-step decisions up to 6 candidates only.
+__device__ __noinline__ void t0_batch(const EnumParams *Pm, WarpSmem *sm, uint32_t nprob) {
+  const uint32_t lane = lane_id();
+  constexpr int NH = kSmallP - 5;
+  uint32_t *ent_leaf = sm->xrow, *ent_sub = sm->xcv;  // the exchange buffer is free inside a solve
+  __syncwarp();
+  const bool live = lane < nprob;
+  const uint32_t P = live ? sm->pr_P[lane] : 0u, RM = live ? sm->pr_RM[lane] : 0u;
+  uint32_t q[5], high = P;
+#pragma unroll
+  for (int k = 0; k < 5; k++) {
+    q[k] = high & (0u - high);
+    high ^= q[k];
+  }
+  // per candidate: the subsets it rules out in a group whose members its row
+  // holds, and the group members its row misses (see t0_small_sets)
+  constexpr uint32_t kWith[5] = {0xAAAAAAAAu, 0xCCCCCCCCu, 0xF0F0F0F0u, 0xFF00FF00u, 0xFFFF0000u};
+  uint32_t dead_in[kSmallP], miss[kSmallP], hb[NH];
+  uint32_t hrest = high;
+#pragma unroll
+  for (int k = 0; k < NH; k++) {
+    hb[k] = hrest & (0u - hrest);
+    hrest ^= hb[k];
+  }
+#pragma unroll
+  for (int i = 0; i < kSmallP; i++) {
+    const uint32_t own = i < 5 ? q[i < 5 ? i : 0] : hb[i < 5 ? 0 : i - 5];
+    const uint32_t row = own ? sm->pr_row[33 * i + lane] : 0u;
+    uint32_t sub = 1;
+#pragma unroll
+    for (int k = 0; k < 5; k++)
+      if (row & q[k]) sub |= sub << (1 << k);
+    dead_in[i] = i < 5 ? sub | (kWith[i < 5 ? i : 0] & ~(sub << (1 << (i < 5 ? i : 0)))) : sub;
+    if (!own) dead_in[i] = 0;
+    miss[i] = own ? high & ~row & ~own : 0u;
+  }
+  const uint32_t n = __popc(P);
+  const uint32_t all = n >= 5 ? 0xffffffffu : live ? (1u << (1u << n)) - 1 : 0u;
+  uint32_t members = 0, queued = 0;
+  bool more = live;
+#pragma unroll 1
+  do {
+    uint32_t dead = 0;
+#pragma unroll
+    for (int i = 0; i < 5; i++) dead |= (members & miss[i]) ? kWith[i] : dead_in[i];
+#pragma unroll
+    for (int k = 0; k < NH; k++) {
+      const uint32_t w = (members & miss[5 + k]) ? 0u : dead_in[5 + k];
+      dead |= (members & hb[k]) ? ~w : w;
+    }
+    uint32_t E = more ? all & ~dead : 0u;
+    const uint32_t fixed = RM | members;
+    for (uint32_t bal = __ballot_sync(kFull, E != 0); bal; bal = __ballot_sync(kFull, E != 0)) {
+      const bool out = E != 0;
+      const uint32_t pos = queued + __popc(bal & lanemask_lt());
+      const uint32_t sub = lane << 5 | (__ffs(E) - 1);
+      E &= E - 1;
+      if (out && pos < 32) {
+        ent_leaf[pos] = fixed;
+        ent_sub[pos] = sub;
       }
-      for (uint32_t k = 0; k < ne; k++) {
-        if (lane == 0) sm->pend_rm[npend] = emit_rm[k];
-        if (++npend == 32) {
-          t0_flush(c, 32, s10, s20, rsize0);
-          npend = 0;
+      queued += __popc(bal);
+      if (queued >= 32) {
+        __syncwarp();
+        t0_hash(Pm, sm, batch_leaf(sm, ent_leaf[lane], ent_sub[lane]), true);
+        if (out && pos >= 32) {
+          ent_leaf[pos - 32] = fixed;
+          ent_sub[pos - 32] = sub;
         }
+        queued -= 32;
       }
-      return;
     }
-  }
-  switch (__popc(P)) {
-    case 3: t0_small_n<3>(c, t, P, A, RM, npend, s10, s20, rsize0); break;
-    case 4: t0_small_n<4>(c, t, P, A, RM, npend, s10, s20, rsize0); break;
-#if MCE_SMALL_P >= 6
-    case 5: t0_small_n<5>(c, t, P, A, RM, npend, s10, s20, rsize0); break;
-#endif
-#if MCE_SMALL_P >= 7
-    case 6: t0_small_n<6>(c, t, P, A, RM, npend, s10, s20, rsize0); break;
-#endif
-    default: t0_small_n<kSmallP < 3 ? 3 : kSmallP>(c, t, P, A, RM, npend, s10, s20, rsize0); break;
+    members = (members - high) & high;
+    more = more && members;
+  } while (__any_sync(kFull, more));
+  __syncwarp();
+  if (queued) {
+    const bool have = lane < queued;
+    t0_hash(Pm, sm, have ? batch_leaf(sm, ent_leaf[lane], ent_sub[lane]) : 0u, have);
   }
 }
+
+// A subproblem that collected fewer small nodes than this decides them one at
+// a time: a batch costs as much for one node as for 32.
+constexpr uint32_t kBatchMin = 16;
 
 // ------------------------------------------------ join decomposition
 // A node whose active rows are all candidates (no X row contains R) has as
@@ -726,8 +763,9 @@ __device__ __forceinline__ void t0_small(const Ctx &c, const T0 &t, uint32_t P, 
 // decided without a search tree: count, histogram and largest size in closed
 // form, and the checksum by walking the products, 32 lanes at a time.
 //
-// Components: breadth-first search with ballots (closed H-neighbourhoods
-// nb = P \ row).  Component j's maximal independent sets come from the 2^s
+// The caller has checked that no closed H-neighbourhood P \ row is larger than
+// a component may be.  Components: breadth-first search with ballots over
+// those.  Component j's maximal independent sets come from the 2^s
 // subsets of its s members, one per lane, and are packed into a table of at
 // most 32 entries in shared memory (hash sums and size of each set).  Lane j
 // holds component j's first entry and entry count.
@@ -742,13 +780,10 @@ constexpr int kJoinComp = 5;    // largest component decided this way
 #endif
 constexpr int kJoinMin = MCE_JOIN_MIN;  // smallest |P| worth the decomposition
 
-__device__ __noinline__ bool t0_join(Ctx c, T0 t, uint32_t P, uint32_t RM, uint64_t s10, uint64_t s20,
-                                     uint32_t rsize0) {
-  const uint32_t lane = c.lane;
-  WarpSmem *sm = c.sm;
+__device__ __noinline__ bool t0_join(const EnumParams *Pm, WarpSmem *sm, uint32_t row, uint32_t P, uint32_t RM) {
+  const uint32_t lane = lane_id();
   const bool inP = (P >> lane) & 1;
-  const uint32_t nb = inP ? (P & ~t.row) : 0u;  // closed non-neighbourhood in P (rows carry no self bit)
-  if (__reduce_max_sync(kFull, (uint32_t)__popc(nb)) > (uint32_t)kJoinComp) return false;
+  const uint32_t nb = inP ? (P & ~row) : 0u;  // closed non-neighbourhood in P (rows carry no self bit)
   const uint32_t single = __ballot_sync(kFull, inP && nb == (1u << lane));  // adjacent to every candidate
   // components first: a node is abandoned before any set is built
   uint32_t rem = P & ~single;
@@ -824,9 +859,9 @@ __device__ __noinline__ bool t0_join(Ctx c, T0 t, uint32_t P, uint32_t RM, uint6
   __syncwarp();
   // the part every clique shares: R and the candidates adjacent to all others
   const uint32_t base_cols = RM | single;
-  const uint64_t b1 = s10 + warp_sum_u64(((base_cols >> lane) & 1) ? t.h1 : 0);
-  const uint64_t b2 = s20 + warp_sum_u64(((base_cols >> lane) & 1) ? t.h2 : 0);
-  const uint32_t size0 = rsize0 + 2 + __popc(base_cols);
+  const uint64_t b1 = sm->t0_s1 + warp_sum_u64(((base_cols >> lane) & 1) ? sm->xh1[lane] : 0);
+  const uint64_t b2 = sm->t0_s2 + warp_sum_u64(((base_cols >> lane) & 1) ? sm->xh2[lane] : 0);
+  const uint32_t size0 = sm->t0_rsize + 2 + __popc(base_cols);
   // sizes: the product of the components' size polynomials, lane = size - size0
   // (a component's sets leave out at least one member, so sizes stay below size0 + 32)
   uint32_t poly = lane == 0 ? 1u : 0u;
@@ -848,9 +883,8 @@ __device__ __noinline__ bool t0_join(Ctx c, T0 t, uint32_t P, uint32_t RM, uint6
       if (size < kHistCache) {
         atomicAdd(&sm->hcache[size], poly);
       } else {
-        const EnumParams &Pm = *c.P;
-        const uint32_t bin = size < Pm.hist_len ? size : Pm.hist_len - 1;
-        atomicAdd(&Pm.hist[(uint64_t)sm->slot * Pm.hist_len + bin], (unsigned long long)poly);
+        const uint32_t bin = size < Pm->hist_len ? size : Pm->hist_len - 1;
+        atomicAdd(&Pm->hist[(uint64_t)sm->slot * Pm->hist_len + bin], (unsigned long long)poly);
       }
     }
     const uint32_t mx = __reduce_max_sync(kFull, poly ? size : 0u);
@@ -918,7 +952,6 @@ __device__ __noinline__ bool t0_join(Ctx c, T0 t, uint32_t P, uint32_t RM, uint6
   }
   sm->lchk[lane] += chk;
   __syncwarp();
-  maybe_flush(c);
   return true;
 }
 
@@ -929,32 +962,25 @@ __device__ __noinline__ bool t0_join(Ctx c, T0 t, uint32_t P, uint32_t RM, uint6
 // work it steps out instead: it saves its state and returns true; the caller
 // (t0_run) exposes levels and calls it again with resume set.
 template <bool kStats>
-__device__ __noinline__ bool t0_solve_body(Ctx c, T0 t, uint32_t pc, uint32_t nrows, uint32_t rsize0, uint64_t s10,
-                                           uint64_t s20, bool resume) {
+__device__ __noinline__ bool t0_solve_body(Ctx c, uint32_t row, uint32_t pc, uint32_t nrows, bool resume) {
   const uint32_t lane = c.lane;
   WarpSmem *sm = c.sm;
   const bool expand_r = c.P->expand_r != 0;
-  uint32_t A, P, RM, npend;
+  uint32_t A, P, RM, npend, nprob;
   int level;
   if (!resume) {
-    sm->xh1[lane] = t.h1;
-    sm->xh2[lane] = t.h2;
-    if (lane == 0) {
-      sm->t0_s1 = s10;
-      sm->t0_s2 = s20;
-      sm->t0_rsize = rsize0;
-    }
-    __syncwarp();
     A = nrows >= 32 ? ~0u : ((1u << nrows) - 1);
     P = pc >= 32 ? ~0u : ((1u << pc) - 1);
     RM = 0;
     npend = 0;
+    nprob = 0;
     level = 0;
   } else {
     P = sm->y_P;
     A = sm->y_A;
     RM = sm->y_RM;
     npend = sm->y_npend;
+    nprob = sm->y_nprob;
     level = sm->y_level;
   }
   const uint32_t lanebit = 1u << lane;
@@ -964,6 +990,7 @@ __device__ __noinline__ bool t0_solve_body(Ctx c, T0 t, uint32_t pc, uint32_t nr
   // A child whose candidate set comes out empty is a leaf: it is tested where
   // it is made, without a frame push, a descent and a backtrack.
   uint32_t VP = 0;
+  uint32_t sP = 0, sA = 0, sRM = 0;  // a node or child that is decided in one step
 node:  // a node with candidates P, active rows A and R = RM
   if (kStats) nodes++;
   if (P == 0) {  // only a subproblem without columns starts like this
@@ -975,16 +1002,23 @@ node:  // a node with candidates P, active rows A and R = RM
   }
   if (__popc(P) <= kSmallP) {
     if (kStats) nodes++;
-    t0_small(c, t, P, A, RM, npend, s10, s20, rsize0);
-    goto backtrack;
+    sP = P;
+    sA = A;
+    sRM = RM;
+    P = 0;  // no candidate of this node is left: the way on is back
+    goto small;
   }
-  if (__popc(P) >= kJoinMin && (A & ~P) == 0 && t0_join(c, t, P, RM, s10, s20, rsize0)) goto backtrack;
   {
-    const uint32_t key = (A & lanebit) ? (((uint32_t)__popc(P & ~t.row) << 5) | lane) : 0xffffffffu;
+    const uint32_t far = (uint32_t)__popc(P & ~row);  // a candidate's row holds no self bit: it counts itself
+    if (__popc(P) >= kJoinMin && (A & ~P) == 0 &&
+        __reduce_max_sync(kFull, (P & lanebit) ? far : 0u) <= (uint32_t)kJoinComp &&
+        t0_join(c.P, sm, row, P, RM))
+      goto backtrack;
+    const uint32_t key = (A & lanebit) ? ((far << 5) | lane) : 0xffffffffu;
     const uint32_t kmin = __reduce_min_sync(kFull, key);
     if (kStats) wops += 2 * __popc(A);  // ANDN + POPC per active row
     if ((kmin >> 5) == 0) goto backtrack;  // an X row covers P: nothing maximal below
-    VP = P & ~__shfl_sync(kFull, t.row, kmin & 31);
+    VP = P & ~__shfl_sync(kFull, row, kmin & 31);
   }
 expand:  // next candidate of VP at this level
   {
@@ -994,18 +1028,18 @@ expand:  // next candidate of VP at this level
     P &= ~(1u << q);
     // the child's candidates and the rows holding q: two independent
     // collectives; rows holding R' = R + q (+ E) are A & those
-    uint32_t P2 = P & __shfl_sync(kFull, t.row, q);
-    uint32_t A2 = A & __ballot_sync(kFull, (t.row >> q) & 1);
+    uint32_t P2 = P & __shfl_sync(kFull, row, q);
+    uint32_t A2 = A & __ballot_sync(kFull, (row >> q) & 1);
     uint32_t M = 1u << q;
     if (expand_r && (P2 & (P2 - 1))) {
       // EXPAND_R: a candidate adjacent to every other candidate joins R at
       // once; rows carry no self bit, so that is P2 \ row == {itself}
-      const uint32_t E = __ballot_sync(kFull, (P2 & ~t.row) == lanebit);
+      const uint32_t E = __ballot_sync(kFull, (P2 & ~row) == lanebit);
       if (kStats) wops += 2 * __popc(P2);
       if (E) {
         P2 &= ~E;
         M |= E;
-        A2 &= __ballot_sync(kFull, (t.row & E) == E);
+        A2 &= __ballot_sync(kFull, (row & E) == E);
       }
     }
     if (kStats) wops += __popc(A) + 1;
@@ -1014,7 +1048,7 @@ expand:  // next candidate of VP at this level
       if (A2 == 0) {
         if (lane == 0) sm->pend_rm[npend] = RM | M;
         if (++npend == 32) {
-          t0_flush(c, 32, s10, s20, rsize0);
+          t0_flush(c, 32);
           npend = 0;
         }
       }
@@ -1022,8 +1056,10 @@ expand:  // next candidate of VP at this level
     }
     if (__popc(P2) <= kSmallP) {  // small child: decided here, no descent
       if (kStats) nodes++;
-      t0_small(c, t, P2, A2, RM | M, npend, s10, s20, rsize0);
-      goto expand;
+      sP = P2;
+      sA = A2;
+      sRM = RM | M;
+      goto small;
     }
     // a child that is its parent's last open candidate replaces the parent
     // (no frame: the parent would only backtrack after it)
@@ -1044,6 +1080,7 @@ expand:  // next candidate of VP at this level
           sm->y_A = A;
           sm->y_RM = RM;
           sm->y_npend = npend;
+          sm->y_nprob = nprob;
           sm->y_level = level;
           if (kStats) {
             sm->nodes += nodes;
@@ -1056,6 +1093,35 @@ expand:  // next candidate of VP at this level
     }
     goto node;
   }
+small:  // one copy of the small decisions, for nodes and children
+  if ((sP & (sP - 1)) == 0) {
+    // One candidate q: R + q is maximal iff no active row holds q (the pivot
+    // step would prune on such a row, else branch on q into a leaf).
+    if ((sA & __ballot_sync(kFull, (row & sP) != 0)) == 0) {
+      if (lane == 0) sm->pend_rm[npend] = sRM | sP;
+      if (++npend == 32) {
+        t0_flush(c, 32);
+        npend = 0;
+      }
+    }
+    goto expand;
+  }
+  // X rows without a candidate rule nothing out
+  if ((sA & ~sP) == 0 || !__any_sync(kFull, (sA & ~sP & lanebit) && (row & sP))) {
+    if (sP & lanebit) sm->pr_row[33 * __popc(sP & lanemask_lt()) + nprob] = row;
+    if (lane == 0) {
+      sm->pr_P[nprob] = sP;
+      sm->pr_RM[nprob] = sRM;
+    }
+    if (++nprob == 32) {
+      t0_batch(c.P, sm, 32);
+      nprob = 0;
+    }
+    goto expand;
+  }
+sets:
+  t0_small_sets(c, row, sP, sA, sRM, npend);
+  goto expand;
 backtrack:
   if (level > 0) {
     level--;
@@ -1066,7 +1132,17 @@ backtrack:
     RM = f.w;
     goto expand;
   }
-  if (npend) t0_flush(c, npend, s10, s20, rsize0);
+  if (nprob >= kBatchMin) {
+    t0_batch(c.P, sm, nprob);
+  } else if (nprob) {  // too few for a batch: one at a time
+    __syncwarp();
+    nprob--;
+    sP = sA = sm->pr_P[nprob];
+    sRM = sm->pr_RM[nprob];
+    P = VP = 0;
+    goto sets;
+  }
+  if (npend) t0_flush(c, npend);
   if (kStats && lane == 0) {
     sm->nodes += nodes;
     sm->wops += wops;
@@ -1078,10 +1154,19 @@ backtrack:
 
 __device__ __forceinline__ void t0_run(const Ctx &c, const T0 &t, uint32_t pc, uint32_t nrows, uint32_t rsize0,
                                        uint64_t s10, uint64_t s20) {
+  WarpSmem *sm = c.sm;
+  sm->xh1[c.lane] = t.h1;
+  sm->xh2[c.lane] = t.h2;
+  if (c.lane == 0) {
+    sm->t0_s1 = s10;
+    sm->t0_s2 = s20;
+    sm->t0_rsize = rsize0;
+  }
+  __syncwarp();
   bool resume = false;
   for (;;) {
-    const bool out = c.P->stats ? t0_solve_body<true>(c, t, pc, nrows, rsize0, s10, s20, resume)
-                                : t0_solve_body<false>(c, t, pc, nrows, rsize0, s10, s20, resume);
+    const bool out = c.P->stats ? t0_solve_body<true>(c, t.row, pc, nrows, resume)
+                                : t0_solve_body<false>(c, t.row, pc, nrows, resume);
     if (!out) break;
     const bool any = t0_share(c, t, c.sm->y_level);
     if (c.lane == 0) c.sm->share_period = any ? kShareMin : min(c.sm->share_period * 2, kShareMax);
