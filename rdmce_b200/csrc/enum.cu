@@ -123,6 +123,7 @@ struct Gen {
   const uint32_t *colv;
   const uint64_t *h1s, *h2s;
   uint64_t *stack;
+  CPlan *plans;  // W of them, for the task being written
   uint32_t *alist;
   uint64_t alist_cap;
   uint32_t pc, nrows, W;
@@ -189,7 +190,7 @@ constexpr uint32_t kTail = kLocalRec + kT1Area;  // slab bytes reserved at its e
 
 // Slab layout of a general-tier problem (bytes from the slab start).
 struct Layout {
-  uint64_t colv_off, hash_off, rows_off, stack_off, alist_off, need;
+  uint64_t colv_off, hash_off, rows_off, stack_off, plan_off, alist_off, need;
 };
 
 __host__ __device__ __forceinline__ Layout layout_for(uint64_t cand_n, uint32_t pc, uint32_t nrows, uint32_t W) {
@@ -199,7 +200,8 @@ __host__ __device__ __forceinline__ Layout layout_for(uint64_t cand_n, uint32_t 
   L.rows_off = L.hash_off + 16ULL * pc;
   L.stack_off = L.rows_off + 8ULL * (uint64_t)nrows * W;
   // pc + 1 levels, one scratch record past the deepest, one spare
-  L.alist_off = L.stack_off + 8ULL * (uint64_t)(pc + 3) * (3ULL * W + 4);
+  L.plan_off = L.stack_off + 8ULL * (uint64_t)(pc + 3) * (3ULL * W + 4);
+  L.alist_off = L.plan_off + 56ULL * W;  // one compression plan a word (CPlan)
   L.need = L.alist_off + 4ULL * nrows + kTail;
   return L;
 }
@@ -421,15 +423,14 @@ __device__ __forceinline__ uint64_t compress_apply(uint64_t x, const CPlan &p) {
   return x;
 }
 
-// multi-word row compaction: out[0..W') = bits of row[0..W) at mask[0..W)
-__device__ __forceinline__ void compress_row(const uint64_t *row, const uint64_t *mask, uint32_t W, uint64_t *out) {
+// multi-word row compaction: out[0..W') = bits of row[0..W) at the masks of plans[0..W)
+__device__ __forceinline__ void compress_row(const uint64_t *row, const CPlan *plans, uint32_t W, uint64_t *out) {
   uint64_t cur = 0;
   uint32_t cb = 0, wi = 0;
   for (uint32_t w = 0; w < W; w++) {
-    const uint64_t m = mask[w];
-    const uint32_t n = __popcll(m);
+    const uint32_t n = __popcll(plans[w].m);
     if (n == 0) continue;
-    const uint64_t c = compress_apply(row[w], compress_plan(m));
+    const uint64_t c = compress_apply(row[w], plans[w]);
     cur |= c << cb;
     if (cb + n >= 64) {
       out[wi++] = cur;
@@ -1374,6 +1375,23 @@ __device__ __noinline__ void t1_solve_body(Ctx c, T1 t, uint32_t pc, uint32_t nr
         if ((key >> 8) == 0) goto backtrack;  // an X row covers P: nothing maximal below
         VP = P & ~bcast_row(t, key & 0xff);
         fresh = false;
+        if (level == 0 && c.sharing && hungry(c)) {  // as in the general tier
+          const unsigned long long ts = now();
+          if (!spawn_outer_gen(c)) {
+            if (lane == 0) {
+              ta->fP[0] = P;
+              ta->fVP[0] = VP;
+              ta->frs[0] = rsize;
+              ta->fs1[0] = s1;
+              ta->fs2[0] = s2;
+            }
+            ta->fab[0][lane] = (uint8_t)ab;
+            __syncwarp();
+            t1_spawn(c, t, 1);
+            VP = ta->fVP[0];
+          }
+          if (lane == 0) sm->cyc[kCycSpawn] += now() - ts;
+        }
       }
     }
     {
@@ -1591,19 +1609,10 @@ __device__ bool gen_materialize(const Ctx &c, const Gen &G, const uint64_t *rec_
       if (row[w] & CP[w]) return true;
     return false;
   };
-  uint32_t nx = 0;
-  for (uint32_t base = 0; base < alen; base += 32) {
-    const uint32_t t = base + lane;
-    bool x = false;
-    if (t < alen) {
-      const uint32_t i = aoff == kIdent ? t : G.alist[aoff + t];
-      x = !is_col(i) && keep_row(i) && hits(i);
-    }
-    nx += __popc(__ballot_sync(kFull, x));
-  }
-  const uint32_t nrows = pc + nx;
-  if (task_bytes(pc, nrows, Wn) > max_bytes) return false;
-  if (to_pool && layout_for(pc, pc, nrows, Wn).need > c.slab_bytes) return false;
+  if (task_bytes(pc, pc, Wn) > max_bytes) return false;
+  // the plans depend on the columns alone: one word a lane, once for the task
+  for (uint32_t w = lane; w < W; w += 32) G.plans[w] = compress_plan(CP[w]);
+  __syncwarp();
   uint32_t *colv = (uint32_t *)(out + kHdr);
   uint64_t *rows = (uint64_t *)(out + kHdr + align8(4ULL * pc));
   // child columns: parent candidate rows i < pc with CP bit i, in order
@@ -1613,7 +1622,7 @@ __device__ bool gen_materialize(const Ctx &c, const Gen &G, const uint64_t *rec_
       for (uint32_t w = 0; w < (i >> 6); w++) k += __popcll(CP[w]);
       k += __popcll(CP[i >> 6] & ((1ULL << (i & 63)) - 1));
       colv[k] = G.colv[i];
-      compress_row(G.rows + (uint64_t)i * W, CP, W, rows + (uint64_t)k * Wn);
+      compress_row(G.rows + (uint64_t)i * W, G.plans, W, rows + (uint64_t)k * Wn);
     }
   }
   uint32_t pos = pc;
@@ -1626,9 +1635,12 @@ __device__ bool gen_materialize(const Ctx &c, const Gen &G, const uint64_t *rec_
       x = !is_col(i) && keep_row(i) && hits(i);
     }
     const uint32_t bal = __ballot_sync(kFull, x);
-    if (x) compress_row(G.rows + (uint64_t)i * W, CP, W, rows + (uint64_t)(pos + __popc(bal & lanemask_lt())) * Wn);
+    if (task_bytes(pc, pos + __popc(bal), Wn) > max_bytes) return false;
+    if (x) compress_row(G.rows + (uint64_t)i * W, G.plans, W, rows + (uint64_t)(pos + __popc(bal & lanemask_lt())) * Wn);
     pos += __popc(bal);
   }
+  const uint32_t nrows = pos;
+  if (to_pool && layout_for(pc, pc, nrows, Wn).need > c.slab_bytes) return false;
   if (lane == 0) {
     TaskHdr *h = (TaskHdr *)out;
     h->pc = pc;
@@ -1793,6 +1805,13 @@ __device__ __noinline__ void gen_solve_body(Ctx c, Gen G, uint32_t rsize0, uint6
       for (uint32_t w = lane; w < W; w += 32) VP[w] = Pv[w] & ~prow[w];
       __syncwarp();
       fresh = false;
+      // idle warps wait for the top of this subproblem's tree: offer it before
+      // the first child, not after eight
+      if (level == 0 && c.sharing && hungry(c)) {
+        const unsigned long long ts = now();
+        gen_spawn(c, G, 1);
+        if (lane == 0) sm->cyc[kCycSpawn] += now() - ts;
+      }
       continue;
     }
     uint32_t q = 0xffffffffu;
@@ -2337,6 +2356,7 @@ __device__ __noinline__ void solve_ego(Ctx c, const uint32_t *colv, uint32_t nro
   G.h1s = h1s;
   G.h2s = h2s;
   G.stack = (uint64_t *)(c.slab + L.stack_off);
+  G.plans = (CPlan *)(c.slab + L.plan_off);
   G.alist = (uint32_t *)(c.slab + L.alist_off);
   G.alist_cap = (c.slab_bytes - kTail - L.alist_off) / 4;
   G.pc = p;
@@ -2500,6 +2520,7 @@ __device__ __noinline__ void solve_block(Ctx c, uint32_t blk) {
   G.h1s = h1s;
   G.h2s = h2s;
   G.stack = (uint64_t *)(c.slab + L.stack_off);
+  G.plans = (CPlan *)(c.slab + L.plan_off);
   G.alist = (uint32_t *)(c.slab + L.alist_off);
   G.alist_cap = (c.slab_bytes - kTail - L.alist_off) / 4;
   G.pc = pc;
