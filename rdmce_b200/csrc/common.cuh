@@ -106,8 +106,9 @@ mce_status scan_exclusive_u32(const uint32_t *in, uint32_t *out, uint64_t n, uin
                               cudaStream_t st);
 mce_status scan_exclusive_u64(const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *d_total,
                               cudaStream_t st);
-// LSD radix sort of n 64-bit keys over bits [0, bits); result in *keys (tmp = scratch of n)
-mce_status radix_sort_u64(uint64_t *keys, uint64_t *tmp, uint64_t n, int bits, cudaStream_t st);
+// stable LSD radix sort of n 64-bit keys by bits [lo, hi) (a last digit may reach past hi: the bits
+// there are zero); tmp = scratch of n, swapped with keys so that the result is in keys
+mce_status radix_sort_u64(uint64_t *&keys, uint64_t *&tmp, uint64_t n, int lo, int hi, cudaStream_t st);
 // allocation-free CSR offsets: off[0..n] = exclusive scan of deg, off[n] = total;
 // partial sums in a fixed device array (n <= 2^26); calls on one device must not overlap
 mce_status csr_offsets_static(int device, const uint32_t *deg, uint32_t *off, uint64_t n, cudaStream_t st);

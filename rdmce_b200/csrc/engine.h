@@ -31,14 +31,13 @@ struct DeviceGraph {
 
 mce_status build_from_pairs(const uint32_t *u_d, const uint32_t *v_d, uint64_t np, int order_kind,
                             uint64_t spin_limit, cudaStream_t st, DeviceGraph *g);
-mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32_t *ev, const uint32_t *deg,
-                        const uint32_t *labels0, int order_kind, uint64_t spin_limit, cudaStream_t st,
-                        DeviceGraph *g);
+mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32_t *ev, const uint32_t *labels0,
+                        int order_kind, uint64_t spin_limit, cudaStream_t st, DeviceGraph *g);
 mce_status build_from_csr(uint64_t n, const uint32_t *off_d, const uint32_t *adj_d, const uint32_t *labels_d,
                           int already_ordered, int order_kind, uint32_t degeneracy_hint, uint64_t spin_limit,
                           cudaStream_t st, DeviceGraph *g);
-mce_status csr_to_edges(uint64_t n, const uint32_t *off, const uint32_t *adj, uint64_t m, uint32_t *deg,
-                        uint32_t **eu, uint32_t **ev, cudaStream_t st);
+mce_status csr_to_edges(uint64_t n, const uint32_t *off, const uint32_t *adj, uint64_t m, uint32_t **eu,
+                        uint32_t **ev, cudaStream_t st);
 void free_graph(DeviceGraph *g);
 // Per-graph figures of a union build (build_union).
 struct UnionCounts {

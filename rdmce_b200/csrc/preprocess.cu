@@ -6,20 +6,22 @@
 //   Graph::SortByDegeneracy/ApplyOrder  src/graph.cc:281-306, 54-77
 //   Graph::ConvertToCsr + LoadFromCpu   src/graph.cc:216-236, src/graph_gpu.cu:3-58
 // Steps: pack (min,max) keys -> radix sort -> unique -> mark/scan dense ids ->
-// degrees -> k-core peeling in synchronous rounds (one cooperative launch) ->
-// relabel both edge directions -> radix sort -> CSR offsets by scan -> root
-// list (v0 < v1) by flag+scan.
+// the same edges by (max,min) by a second sort -> degrees and adjacency from
+// the two sorted lists -> k-core peeling in synchronous rounds (one cooperative
+// launch) -> both edge directions under the new ids, already ordered by column
+// -> radix sort by row -> CSR -> root list (v0 < v1) by flag+scan.
+//
+// Every list that is built is a sorted one, so degrees are lengths of runs and
+// places in a row are differences of positions: no counting or cursor atomics,
+// which serialise on the hubs of a skewed graph (R-MAT 20: 3.9 of the build's
+// 14.5 ms on a B200).
 #include <algorithm>
 #include <vector>
-
-#include <cooperative_groups.h>
 
 #include "common.cuh"
 #include "engine.h"
 
 namespace mce {
-
-namespace cg = cooperative_groups;
 
 namespace {
 
@@ -67,25 +69,61 @@ __global__ void k_labels_from_marks(const uint32_t *mark, const uint32_t *id, ui
     if (mark[l]) labels[id[l]] = (uint32_t)l;
 }
 
-// edges (label pair) -> dense ids, degrees
+// edges (label pair) -> dense ids
 __global__ void k_map_edges(uint64_t *edges, uint64_t m, int bits, const uint32_t *id, uint32_t *eu,
-                            uint32_t *ev, uint32_t *deg) {
+                            uint32_t *ev) {
   const uint64_t mask = (1ULL << bits) - 1;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t a = id[edges[i] >> bits], b = id[edges[i] & mask];
-    eu[i] = a;
-    ev[i] = b;
-    atomicAdd(&deg[a], 1u);
-    atomicAdd(&deg[b], 1u);
+    eu[i] = id[edges[i] >> bits];
+    ev[i] = id[edges[i] & mask];
   }
 }
 
-// unsorted symmetric adjacency for peeling
-__global__ void k_fill_adj(const uint32_t *eu, const uint32_t *ev, uint64_t m, uint32_t *cursor, uint32_t *adj) {
+// the edges keyed by (larger id, smaller id)
+__global__ void k_swap_keys(const uint32_t *eu, const uint32_t *ev, uint64_t m, int nb, uint64_t *keys) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
+    keys[i] = ((uint64_t)ev[i] << nb) | eu[i];
+}
+
+// Where each vertex's run begins and ends in the edges by smaller id (eu: its
+// larger neighbours) and by larger id (the keys' rows: its smaller ones);
+// vertices without a run keep begin = end = 0.
+__global__ void k_run_bounds(const uint32_t *eu, const uint64_t *by_v, uint64_t m, int nb, uint32_t *ub, uint32_t *ue,
+                             uint32_t *lb, uint32_t *le) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t a = eu[i], b = ev[i];
-    adj[atomicAdd(&cursor[a], 1u)] = b;
-    adj[atomicAdd(&cursor[b], 1u)] = a;
+    const uint32_t a = eu[i], b = (uint32_t)(by_v[i] >> nb);
+    if (i == 0 || eu[i - 1] != a) ub[a] = (uint32_t)i;
+    if (i == m - 1 || eu[i + 1] != a) ue[a] = (uint32_t)i + 1;
+    if (i == 0 || (uint32_t)(by_v[i - 1] >> nb) != b) lb[b] = (uint32_t)i;
+    if (i == m - 1 || (uint32_t)(by_v[i + 1] >> nb) != b) le[b] = (uint32_t)i + 1;
+  }
+}
+
+__global__ void k_run_degrees(const uint32_t *ub, const uint32_t *ue, const uint32_t *lb, const uint32_t *le,
+                              uint32_t n, uint32_t *deg) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+    deg[v] = (ue[v] - ub[v]) + (le[v] - lb[v]);
+}
+
+// Row r of vertex v starts at off[r]; its smaller neighbours come first.  The
+// element at position i of a sorted edge list goes to i + (the list's base of
+// v), modulo 2^32.
+__global__ void k_run_bases(const uint32_t *off, const uint32_t *rank, const uint32_t *ub, const uint32_t *lb,
+                            const uint32_t *le, uint32_t n, uint32_t *ubase, uint32_t *lbase) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const uint32_t o = off[rank ? rank[v] : v];
+    lbase[v] = o - lb[v];
+    ubase[v] = o + (le[v] - lb[v]) - ub[v];
+  }
+}
+
+// symmetric adjacency for peeling
+__global__ void k_fill_adj(const uint32_t *eu, const uint32_t *ev, const uint64_t *by_v, uint64_t m, int nb,
+                           const uint32_t *ubase, const uint32_t *lbase, uint32_t *adj) {
+  const uint64_t mask = (1ULL << nb) - 1;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
+    adj[ubase[eu[i]] + (uint32_t)i] = ev[i];
+    adj[lbase[by_v[i] >> nb] + (uint32_t)i] = (uint32_t)(by_v[i] & mask);
   }
 }
 
@@ -106,25 +144,57 @@ __global__ void k_iota(uint32_t *a, uint64_t n) {
 // (edges of the ordered CSR) are stable from run to run; the reference's
 // sequential queue (graph.cc:289-304) orders vertices inside a round
 // differently, which changes neither the degeneracy nor the clique set.
+// A skewed graph's core peels in hundreds of levels of a few rounds each, with
+// little work in most: the time is barriers and dependent L2 accesses.  So
+// counters are never reused (one per round and per level, cleared up front),
+// which leaves one barrier a scan and one a round; the barrier is one counter
+// that 148 blocks add to; and a warp keeps four neighbours in flight.
+// Measured (B200): R-MAT 20 (192 levels, 622 rounds) 5.3 -> 4.4 ms.
 struct PeelCtl {
-  uint32_t fcnt[3];     // frontier sizes, by round mod 3
-  uint32_t rcnt[3];     // survivors of each level's scan, by level mod 3
-  uint32_t rmin[3];     // smallest surviving residual degree, by level mod 3
+  uint32_t arrived;     // barrier arrivals so far
   uint32_t degeneracy;
   uint32_t rounds;
   uint32_t levels;
-  uint32_t error;       // 1: level bound exceeded (cannot happen on a consistent CSR)
+  uint32_t error;       // 1: level bound exceeded (cannot happen on a consistent CSR); 2: a barrier wait ran out
 };
+constexpr uint32_t kPeelThreads = 512;
 
-__global__ void __launch_bounds__(256) k_peel_rounds(uint32_t n, const uint32_t *off, const uint32_t *adj,
-                                                     int *deg, uint32_t *state, uint32_t *remA, uint32_t *remB,
-                                                     uint32_t *frA, uint32_t *frB, PeelCtl *ctl, uint32_t max_levels) {
-  cg::grid_group grid = cg::this_grid();
+// One barrier of the whole grid (all blocks are resident); false when the wait
+// ran out.
+__device__ __forceinline__ bool grid_barrier(PeelCtl *ctl, uint32_t *target, uint64_t spin_limit) {
+  __shared__ uint32_t ok;
+  *target += gridDim.x;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicAdd(&ctl->arrived, 1u);
+    uint32_t seen = 0;
+    uint64_t n = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&ctl->arrived) : "memory");
+    } while (seen < *target && ++n < spin_limit);
+    ok = seen >= *target;
+    if (!ok) atomicExch(&ctl->error, 2u);
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// fcnt[r]: vertices claimed into round r; rcnt[l], rmin[l]: survivors of level
+// l's scan and their smallest residual degree.
+__global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const uint32_t *off, const uint32_t *adj,
+                                                              int *deg, uint32_t *state, uint32_t *remA,
+                                                              uint32_t *remB, uint32_t *frA, uint32_t *frB,
+                                                              PeelCtl *ctl, uint32_t *fcnt, uint32_t *rcnt,
+                                                              uint32_t *rmin, uint32_t max_levels,
+                                                              uint64_t spin_limit) {
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t gwarp = tid >> 5, nwarps = nthreads >> 5;
   const bool leader = tid == 0;
+  uint32_t target = 0;
   uint32_t k = 0, degen = 0, lev = 0, r = 0, removed = 0, nrem = n;
   uint32_t *rem_cur = remA, *rem_nxt = remB;
   while (removed < n) {
@@ -134,10 +204,6 @@ __global__ void __launch_bounds__(256) k_peel_rounds(uint32_t n, const uint32_t 
     }
     uint32_t *fr = (r & 1) ? frB : frA;
     // scan: claim residual degree <= k into F_r, keep the rest
-    if (leader) {
-      ctl->rcnt[(lev + 1) % 3] = 0;
-      ctl->rmin[(lev + 1) % 3] = 0xffffffffu;
-    }
     uint32_t local_min = 0xffffffffu;
     // warp-uniform trip count; one atomic per warp and list (every survivor
     // is appended at every level, so per-thread atomics on one counter would
@@ -149,8 +215,8 @@ __global__ void __launch_bounds__(256) k_peel_rounds(uint32_t n, const uint32_t 
       bool claim = false, keep = false;
       if (i < nrem) {
         v = __ldcg(rem_cur + i);
+        d = __ldcg(deg + v);
         if (!__ldcg(state + v)) {
-          d = __ldcg(deg + v);
           claim = d <= (int)k;
           keep = !claim;
         }
@@ -158,8 +224,8 @@ __global__ void __launch_bounds__(256) k_peel_rounds(uint32_t n, const uint32_t 
       const uint32_t cm = __ballot_sync(kFull, claim), km = __ballot_sync(kFull, keep);
       uint32_t cb = 0, kb = 0;
       if (lane == 0) {
-        if (cm) cb = atomicAdd(&ctl->fcnt[r % 3], (uint32_t)__popc(cm));
-        if (km) kb = atomicAdd(&ctl->rcnt[lev % 3], (uint32_t)__popc(km));
+        if (cm) cb = atomicAdd(&fcnt[r], (uint32_t)__popc(cm));
+        if (km) kb = atomicAdd(&rcnt[lev], (uint32_t)__popc(km));
       }
       cb = __shfl_sync(kFull, cb, 0);
       kb = __shfl_sync(kFull, kb, 0);
@@ -172,17 +238,16 @@ __global__ void __launch_bounds__(256) k_peel_rounds(uint32_t n, const uint32_t 
       }
     }
     local_min = __reduce_min_sync(kFull, local_min);
-    if (lane == 0 && local_min != 0xffffffffu) atomicMin(&ctl->rmin[lev % 3], local_min);
-    grid.sync();
+    if (lane == 0 && local_min != 0xffffffffu) atomicMin(&rmin[lev], local_min);
+    if (!grid_barrier(ctl, &target, spin_limit)) return;
     uint32_t level_claims = 0;
     for (;;) {
-      const uint32_t nf = __ldcg(&ctl->fcnt[r % 3]);
+      const uint32_t nf = __ldcg(&fcnt[r]);
       if (nf == 0) break;
       level_claims += nf;
       removed += nf;
       const uint32_t *cur = (r & 1) ? frB : frA;
       uint32_t *nxt = (r & 1) ? frA : frB;
-      if (leader) ctl->fcnt[(r + 2) % 3] = 0;  // last read in round r - 1
       // Each frontier vertex's adjacency is shared by `per` warps (all the
       // grid's warps split evenly when the frontier is small: the dense
       // cores' hubs hold tens of thousands of neighbours each).
@@ -191,21 +256,36 @@ __global__ void __launch_bounds__(256) k_peel_rounds(uint32_t n, const uint32_t 
         const uint32_t v = __ldcg(cur + i);
         const uint32_t e1 = off[v + 1];
         const uint32_t part = (uint32_t)(gwarp % per);
-        for (uint64_t e = (uint64_t)off[v] + 32ULL * part + lane; e < e1; e += 32ULL * per) {
-          const uint32_t u = adj[e];
-          if (__ldcg(state + u)) continue;
-          if (atomicSub(&deg[u], 1) == (int)k + 1 && atomicCAS(&state[u], 0u, r + 2) == 0u)
-            nxt[atomicAdd(&ctl->fcnt[(r + 1) % 3], 1u)] = u;
+        const uint64_t step = 32ULL * per;
+        for (uint64_t e = (uint64_t)off[v] + 32ULL * part + lane; e < e1; e += 4 * step) {
+          uint32_t u[4];
+          bool open[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            open[j] = e + j * step < e1;
+            u[j] = open[j] ? adj[e + j * step] : 0;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; j++) open[j] = open[j] && !__ldcg(state + u[j]);
+          int was[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) was[j] = open[j] ? atomicSub(&deg[u[j]], 1) : 0;
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (open[j] && was[j] == (int)k + 1) {  // one decrement alone sees k + 1: it claims the vertex
+              state[u[j]] = r + 2;
+              nxt[atomicAdd(&fcnt[r + 1], 1u)] = u[j];
+            }
         }
       }
-      grid.sync();
+      if (!grid_barrier(ctl, &target, spin_limit)) return;
       r++;
     }
     // F_r is empty: round index r is skipped, so no vertex of the next level
     // shares a round number with this level's
     r++;
-    nrem = __ldcg(&ctl->rcnt[lev % 3]);
-    const uint32_t rmin = __ldcg(&ctl->rmin[lev % 3]);
+    nrem = __ldcg(&rcnt[lev]);
+    const uint32_t least = __ldcg(&rmin[lev]);
     uint32_t *t = rem_cur;
     rem_cur = rem_nxt;
     rem_nxt = t;
@@ -213,15 +293,13 @@ __global__ void __launch_bounds__(256) k_peel_rounds(uint32_t n, const uint32_t 
       degen = k;
       k = k + 1;
     } else {
-      if (rmin == 0xffffffffu) break;
-      k = max(k + 1, rmin);
+      if (least == 0xffffffffu) break;
+      k = max(k + 1, least);
     }
     lev++;
-    // The next scan fills fcnt[r % 3] and the round after it fcnt[(r + 1) % 3],
-    // which still holds the size of this level's last processed round; the
-    // only counter still being read (fcnt of the empty round) is already zero.
-    if (leader) ctl->fcnt[0] = ctl->fcnt[1] = ctl->fcnt[2] = 0;
-    grid.sync();
+    // The next scan needs no barrier of its own: the last one above came after
+    // every decrement of this level, and the lists and counters the scan
+    // writes are not read any more.
   }
   if (leader) {
     ctl->degeneracy = degen;
@@ -244,15 +322,21 @@ __global__ void k_rank_from_order(const uint32_t *order, uint32_t n, uint32_t *r
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) rank[order[i]] = i;
 }
 
-// both directions of every edge under the new ids, packed (row << nb) | col
-__global__ void k_relabel_keys(const uint32_t *eu, const uint32_t *ev, uint64_t m, const uint32_t *rank, int nb,
-                               uint64_t *keys, uint32_t *deg_new) {
+__global__ void k_permute_degrees(const uint32_t *deg, const uint32_t *rank, uint32_t n, uint32_t *deg_new) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) deg_new[rank[i]] = deg[i];
+}
+
+// Both directions of every edge under the new ids, packed (row << nb) | col.
+// Vertex v's edges are written with v as the column, in v's new row: the list
+// comes out ordered by column, and a stable sort by row alone finishes it.
+__global__ void k_relabel_keys(const uint32_t *eu, const uint32_t *ev, const uint64_t *by_v, uint64_t m,
+                               const uint32_t *rank, const uint32_t *ubase, const uint32_t *lbase, int nb,
+                               uint64_t *keys) {
+  const uint64_t mask = (1ULL << nb) - 1;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t a = rank[eu[i]], b = rank[ev[i]];
-    keys[2 * i] = ((uint64_t)a << nb) | b;
-    keys[2 * i + 1] = ((uint64_t)b << nb) | a;
-    atomicAdd(&deg_new[a], 1u);
-    atomicAdd(&deg_new[b], 1u);
+    const uint32_t u = eu[i], v = (uint32_t)(by_v[i] >> nb);
+    keys[ubase[u] + (uint32_t)i] = ((uint64_t)rank[ev[i]] << nb) | rank[u];
+    keys[lbase[v] + (uint32_t)i] = ((uint64_t)rank[by_v[i] & mask] << nb) | rank[v];
   }
 }
 
@@ -339,7 +423,7 @@ mce_status read_scalar(const T *d, T *h, cudaStream_t st) {
 
 // k-core peeling over an unsorted symmetric CSR; fills order[] (position -> vertex)
 mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint32_t *deg0, uint32_t max_degree,
-                uint32_t *order, uint32_t *degeneracy, cudaStream_t st) {
+                uint32_t *order, uint32_t *degeneracy, uint64_t spin_limit, cudaStream_t st) {
   DevBuf<int> deg;
   DevBuf<uint32_t> state, remA, remB, frA, frB;
   DevBuf<PeelCtl> ctl;
@@ -353,32 +437,38 @@ mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint
   MCE_CUDA_TRY(cudaMemcpyAsync(deg.p, deg0, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
   MCE_CUDA_TRY(cudaMemsetAsync(state.p, 0, n * sizeof(uint32_t), st));
   k_iota<<<grid_for(n, 256), 256, 0, st>>>(remA.p, n); note_launch();
-  // the control block goes through ordinary host memory: pinning it for each
-  // build (and unpinning, which synchronises the device) would stall other
-  // streams' work, e.g. concurrently served requests
+  // one counter a round (every round but the last of a level claims a vertex)
+  // and two a level
+  const uint64_t max_levels = (uint64_t)max_degree + 2, max_rounds = (uint64_t)n + max_levels + 4;
+  DevBuf<uint32_t> counters;
+  MCE_TRY(counters.alloc(max_rounds + 2 * (max_levels + 2), st));
+  uint32_t *fcnt = counters.p, *rcnt = fcnt + max_rounds, *rmin = rcnt + max_levels + 2;
+  MCE_CUDA_TRY(cudaMemsetAsync(fcnt, 0, (max_rounds + max_levels + 2) * sizeof(uint32_t), st));
+  MCE_CUDA_TRY(cudaMemsetAsync(rmin, 0xff, (max_levels + 2) * sizeof(uint32_t), st));
+  MCE_CUDA_TRY(cudaMemsetAsync(ctl.p, 0, sizeof(PeelCtl), st));
+  // the control block is read through ordinary host memory: pinning it for
+  // each build (and unpinning, which synchronises the device) would stall
+  // other streams' work, e.g. concurrently served requests
   PeelCtl h{};
-  for (int i = 0; i < 3; i++) h.rmin[i] = 0xffffffffu;
-  PeelCtl hc_buf = h;
-  PeelCtl *hc = &hc_buf;
-  MCE_CUDA_TRY(cudaMemcpyAsync(ctl.p, hc, sizeof(PeelCtl), cudaMemcpyHostToDevice, st));
+  PeelCtl *hc = &h;
   int dev = 0, sms = 0, per_sm = 0;
   MCE_CUDA_TRY(cudaGetDevice(&dev));
   MCE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  MCE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel_rounds, 256, 0));
+  MCE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel_rounds, kPeelThreads, 0));
   if (per_sm < 1) return MCE_ERR_INTERNAL;
-  // a cooperative launch: every block is resident, so grid.sync() is sound
-  const uint32_t blocks = (uint32_t)std::min(per_sm, 2) * (uint32_t)sms;
-  uint32_t nn = n, maxl = max_degree + 2;
+  // a cooperative launch: every block is resident, so the barrier is sound
+  const uint32_t blocks = (uint32_t)sms;
+  uint32_t nn = n, maxl = (uint32_t)max_levels;
   int *degp = deg.p;
   uint32_t *statep = state.p, *ra = remA.p, *rb = remB.p, *fa = frA.p, *fb = frB.p;
   PeelCtl *cp = ctl.p;
-  void *args[] = {&nn, (void *)&off, (void *)&adj, &degp, &statep, &ra, &rb, &fa, &fb, &cp, &maxl};
-  MCE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_peel_rounds, dim3(blocks), dim3(256), args, 0, st));
+  void *args[] = {&nn, (void *)&off, (void *)&adj, &degp, &statep, &ra, &rb, &fa, &fb, &cp, &fcnt, &rcnt, &rmin, &maxl,
+                  &spin_limit};
+  MCE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_peel_rounds, dim3(blocks), dim3(kPeelThreads), args, 0, st));
   note_launch();
   MCE_CUDA_TRY(cudaMemcpyAsync(hc, ctl.p, sizeof(PeelCtl), cudaMemcpyDeviceToHost, st));
   MCE_CUDA_TRY(cudaStreamSynchronize(st));
-  h = *hc;
-  if (h.error) return MCE_ERR_INTERNAL;
+  if (h.error) return h.error == 2 ? MCE_ERR_TIMEOUT : MCE_ERR_INTERNAL;
   *degeneracy = h.degeneracy;
   // order = vertices sorted by (round, id)
   const int nb = bits_for(n ? n - 1 : 0), rb_bits = bits_for(h.rounds);
@@ -387,7 +477,8 @@ mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint
   MCE_TRY(keys.alloc(n, st));
   MCE_TRY(tmp.alloc(n, st));
   k_round_keys<<<grid_for(n, 256), 256, 0, st>>>(state.p, n, nb, keys.p); note_launch();
-  MCE_TRY(radix_sort_u64(keys.p, tmp.p, n, nb + rb_bits, st));
+  // the keys are in vertex order already: a stable sort by round finishes them
+  MCE_TRY(radix_sort_u64(keys.p, tmp.p, n, nb, nb + rb_bits, st));
   k_order_from_round_keys<<<grid_for(n, 256), 256, 0, st>>>(keys.p, n, (1ULL << nb) - 1, order); note_launch();
   MCE_CUDA_TRY(cudaGetLastError());
   return MCE_OK;
@@ -437,14 +528,10 @@ __device__ __forceinline__ uint32_t find_label(const uint32_t *labels, uint32_t 
 }
 
 __global__ void k_map_edges_search(const uint64_t *edges, uint64_t m, const uint32_t *labels, uint32_t n,
-                                   uint32_t *eu, uint32_t *ev, uint32_t *deg) {
+                                   uint32_t *eu, uint32_t *ev) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t a = find_label(labels, n, (uint32_t)(edges[i] >> 32));
-    const uint32_t b = find_label(labels, n, (uint32_t)(edges[i] & 0xffffffffULL));
-    eu[i] = a;
-    ev[i] = b;
-    atomicAdd(&deg[a], 1u);
-    atomicAdd(&deg[b], 1u);
+    eu[i] = find_label(labels, n, (uint32_t)(edges[i] >> 32));
+    ev[i] = find_label(labels, n, (uint32_t)(edges[i] & 0xffffffffULL));
   }
 }
 
@@ -456,7 +543,7 @@ mce_status build_sparse_labels(const uint32_t *u, const uint32_t *v, uint64_t np
   MCE_TRY(keys.alloc(np, st));
   MCE_TRY(tmp.alloc(np, st));
   k_pack_keys64<<<grid_for(np, 256), 256, 0, st>>>(u, v, np, keys.p); note_launch();
-  MCE_TRY(radix_sort_u64(keys.p, tmp.p, np, 64, st));
+  MCE_TRY(radix_sort_u64(keys.p, tmp.p, np, 0, 64, st));
   DevBuf<uint32_t> flags, pos;
   MCE_TRY(flags.alloc(np + 1, st));
   MCE_TRY(pos.alloc(np + 1, st));
@@ -478,7 +565,7 @@ mce_status build_sparse_labels(const uint32_t *u, const uint32_t *v, uint64_t np
   MCE_TRY(ends.alloc(k, st));
   MCE_TRY(etmp.alloc(k, st));
   k_endpoints<<<grid_for(m, 256), 256, 0, st>>>(edges.p, m, ends.p); note_launch();
-  MCE_TRY(radix_sort_u64(ends.p, etmp.p, k, 32, st));
+  MCE_TRY(radix_sort_u64(ends.p, etmp.p, k, 0, 32, st));
   etmp.release();
   DevBuf<uint32_t> f2, p2;
   MCE_TRY(f2.alloc(k + 1, st));
@@ -487,19 +574,17 @@ mce_status build_sparse_labels(const uint32_t *u, const uint32_t *v, uint64_t np
   MCE_TRY(scan_exclusive_u32(f2.p, p2.p, k, p2.p + k, st));
   uint32_t n = 0;
   MCE_TRY(read_scalar(p2.p + k, &n, st));
-  DevBuf<uint32_t> labels0, eu, ev, deg;
+  DevBuf<uint32_t> labels0, eu, ev;
   MCE_TRY(labels0.alloc(n, st));
   MCE_TRY(eu.alloc(m, st));
   MCE_TRY(ev.alloc(m, st));
-  MCE_TRY(deg.alloc(n + 1, st));
   k_labels_from_sorted<<<grid_for(k, 256), 256, 0, st>>>(ends.p, f2.p, p2.p, k, labels0.p); note_launch();
-  MCE_CUDA_TRY(cudaMemsetAsync(deg.p, 0, (n + 1) * sizeof(uint32_t), st));
-  k_map_edges_search<<<grid_for(m, 256), 256, 0, st>>>(edges.p, m, labels0.p, n, eu.p, ev.p, deg.p); note_launch();
+  k_map_edges_search<<<grid_for(m, 256), 256, 0, st>>>(edges.p, m, labels0.p, n, eu.p, ev.p); note_launch();
   ends.release();
   f2.release();
   p2.release();
   edges.release();
-  MCE_TRY(finish_graph(n, m, eu.p, ev.p, deg.p, labels0.p, order_kind, spin_limit, st, g));
+  MCE_TRY(finish_graph(n, m, eu.p, ev.p, labels0.p, order_kind, spin_limit, st, g));
   return MCE_OK;
 }
 
@@ -527,7 +612,7 @@ mce_status build_from_pairs(const uint32_t *u, const uint32_t *v, uint64_t np, i
   MCE_TRY(keys.alloc(np, st));
   MCE_TRY(tmp.alloc(np, st));
   k_pack_keys<<<grid_for(np, 256), 256, 0, st>>>(u, v, np, lb, keys.p); note_launch();
-  MCE_TRY(radix_sort_u64(keys.p, tmp.p, np, 2 * lb, st));
+  MCE_TRY(radix_sort_u64(keys.p, tmp.p, np, 0, 2 * lb, st));
   DevBuf<uint32_t> flags, pos;
   MCE_TRY(flags.alloc(np + 1, st));
   MCE_TRY(pos.alloc(np + 1, st));
@@ -555,34 +640,48 @@ mce_status build_from_pairs(const uint32_t *u, const uint32_t *v, uint64_t np, i
   MCE_TRY(scan_exclusive_u32(mark.p, id.p, nl, id.p + nl, st));
   uint32_t n = 0;
   MCE_TRY(read_scalar(id.p + nl, &n, st));
-  DevBuf<uint32_t> labels0, eu, ev, deg;
+  DevBuf<uint32_t> labels0, eu, ev;
   MCE_TRY(labels0.alloc(n, st));
   MCE_TRY(eu.alloc(m, st));
   MCE_TRY(ev.alloc(m, st));
-  MCE_TRY(deg.alloc(n + 1, st));
   k_labels_from_marks<<<grid_for(nl, 256), 256, 0, st>>>(mark.p, id.p, nl, labels0.p); note_launch();
-  MCE_CUDA_TRY(cudaMemsetAsync(deg.p, 0, (n + 1) * sizeof(uint32_t), st));
-  k_map_edges<<<grid_for(m, 256), 256, 0, st>>>(edges.p, m, lb, id.p, eu.p, ev.p, deg.p); note_launch();
+  k_map_edges<<<grid_for(m, 256), 256, 0, st>>>(edges.p, m, lb, id.p, eu.p, ev.p); note_launch();
   mark.release();
   id.release();
   edges.release();
-  MCE_TRY(finish_graph(n, m, eu.p, ev.p, deg.p, labels0.p, order_kind, spin_limit, st, g));
+  MCE_TRY(finish_graph(n, m, eu.p, ev.p, labels0.p, order_kind, spin_limit, st, g));
   return MCE_OK;
 }
 
-// eu/ev: m edges on dense ids (any order, no duplicates, no self-loops);
-// deg: degrees (n); labels0: original labels of the dense ids.
-mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32_t *ev, const uint32_t *deg,
-                        const uint32_t *labels0, int order_kind, uint64_t spin_limit, cudaStream_t st,
-                        DeviceGraph *g) {
+// eu/ev: m edges eu < ev on dense ids, sorted by (eu, ev), without duplicates;
+// labels0: original labels of the dense ids.
+mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32_t *ev, const uint32_t *labels0,
+                        int order_kind, uint64_t spin_limit, cudaStream_t st, DeviceGraph *g) {
   *g = DeviceGraph{};
   g->n = n;
   g->m = m;
   g->stream = st;
   if (2 * m >= (1ULL << 32)) return MCE_ERR_TOO_LARGE;
+  const int nb = bits_for(n ? n - 1 : 0);
+  const uint64_t m2 = 2 * m;
+  // the edges by larger id, and every vertex's runs in both lists
+  DevBuf<uint64_t> by_v, tmp_v;
+  MCE_TRY(by_v.alloc(m, st));
+  MCE_TRY(tmp_v.alloc(m, st));
+  k_swap_keys<<<grid_for(m, 256), 256, 0, st>>>(eu, ev, m, nb, by_v.p); note_launch();
+  MCE_TRY(radix_sort_u64(by_v.p, tmp_v.p, m, nb, 2 * nb, st));
+  tmp_v.release();
+  DevBuf<uint32_t> runs, bases, deg;
+  MCE_TRY(runs.alloc(4ULL * n, st));
+  MCE_TRY(bases.alloc(2ULL * n, st));
+  MCE_TRY(deg.alloc(n + 1, st));
+  uint32_t *ub = runs.p, *ue = ub + n, *lb = ue + n, *le = lb + n, *ubase = bases.p, *lbase = ubase + n;
+  MCE_CUDA_TRY(cudaMemsetAsync(runs.p, 0, 4ULL * n * sizeof(uint32_t), st));
+  k_run_bounds<<<grid_for(m, 256), 256, 0, st>>>(eu, by_v.p, m, nb, ub, ue, lb, le); note_launch();
+  k_run_degrees<<<grid_for(n, 256), 256, 0, st>>>(ub, ue, lb, le, n, deg.p); note_launch();
   DevBuf<uint32_t> maxd;
   MCE_TRY(maxd.alloc(1, st));
-  MCE_TRY(reduce_max_u32(deg, n, maxd.p, st));
+  MCE_TRY(reduce_max_u32(deg.p, n, maxd.p, st));
   MCE_TRY(read_scalar(maxd.p, &g->max_degree, st));
 
   // 3) vertex order
@@ -591,20 +690,19 @@ mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32
   MCE_TRY(rank.alloc(n, st));
   g->degeneracy = g->max_degree;  // Graph::LoadFromFile leaves degeneracy_ = max degree (graph.cc:149)
   if (order_kind == MCE_ORDER_DEGENERACY && n > 0) {
-    DevBuf<uint32_t> off0, cursor, adj0;
+    DevBuf<uint32_t> off0, adj0;
     MCE_TRY(off0.alloc(n + 1, st));
-    MCE_TRY(cursor.alloc(n + 1, st));
-    MCE_TRY(adj0.alloc(2 * m, st));
-    MCE_TRY(scan_exclusive_u32(deg, off0.p, n, off0.p + n, st));
-    MCE_CUDA_TRY(cudaMemcpyAsync(cursor.p, off0.p, (n + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-    k_fill_adj<<<grid_for(m, 256), 256, 0, st>>>(eu, ev, m, cursor.p, adj0.p); note_launch();
-    MCE_TRY(peel(n, off0.p, adj0.p, deg, g->max_degree, order.p, &g->degeneracy, st));
+    MCE_TRY(adj0.alloc(m2, st));
+    MCE_TRY(scan_exclusive_u32(deg.p, off0.p, n, off0.p + n, st));
+    k_run_bases<<<grid_for(n, 256), 256, 0, st>>>(off0.p, nullptr, ub, lb, le, n, ubase, lbase); note_launch();
+    k_fill_adj<<<grid_for(m, 256), 256, 0, st>>>(eu, ev, by_v.p, m, nb, ubase, lbase, adj0.p); note_launch();
+    MCE_TRY(peel(n, off0.p, adj0.p, deg.p, g->max_degree, order.p, &g->degeneracy, spin_limit, st));
   } else if ((order_kind == MCE_ORDER_DEGREE_ASC || order_kind == MCE_ORDER_DEGREE_DESC) && n > 0) {
     DevBuf<uint64_t> dk, dt;
     MCE_TRY(dk.alloc(n, st));
     MCE_TRY(dt.alloc(n, st));
-    k_degree_keys<<<grid_for(n, 256), 256, 0, st>>>(deg, n, order_kind == MCE_ORDER_DEGREE_DESC, dk.p); note_launch();
-    MCE_TRY(radix_sort_u64(dk.p, dt.p, n, 64, st));
+    k_degree_keys<<<grid_for(n, 256), 256, 0, st>>>(deg.p, n, order_kind == MCE_ORDER_DEGREE_DESC, dk.p); note_launch();
+    MCE_TRY(radix_sort_u64(dk.p, dt.p, n, 0, 64, st));
     k_order_from_keys<<<grid_for(n, 256), 256, 0, st>>>(dk.p, n, order.p); note_launch();
   } else {
     k_iota<<<grid_for(n, 256), 256, 0, st>>>(order.p, n); note_launch();
@@ -613,20 +711,20 @@ mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32
   order.release();
 
   // 4) relabelled symmetric edge keys -> sorted CSR
-  const int nb = bits_for(n ? n - 1 : 0);
-  const uint64_t m2 = 2 * m;
   DevBuf<uint64_t> keys, tmp;
   MCE_TRY(keys.alloc(m2, st));
   MCE_TRY(tmp.alloc(m2, st));
   DevBuf<uint32_t> deg_new;
   MCE_TRY(deg_new.alloc(n + 1, st));
-  MCE_CUDA_TRY(cudaMemsetAsync(deg_new.p, 0, (n + 1) * sizeof(uint32_t), st));
-  k_relabel_keys<<<grid_for(m, 256), 256, 0, st>>>(eu, ev, m, rank.p, nb, keys.p, deg_new.p); note_launch();
-  MCE_TRY(radix_sort_u64(keys.p, tmp.p, m2, 2 * nb, st));
-  tmp.release();
+  k_permute_degrees<<<grid_for(n, 256), 256, 0, st>>>(deg.p, rank.p, n, deg_new.p); note_launch();
   MCE_CUDA_TRY(cudaMallocAsync(&g->off, (n + 1) * sizeof(uint32_t), st));
-  MCE_CUDA_TRY(cudaMallocAsync(&g->adj, std::max<uint64_t>(m2, 1) * sizeof(uint32_t), st));
   MCE_TRY(scan_exclusive_u32(deg_new.p, g->off, n, g->off + n, st));
+  k_run_bases<<<grid_for(n, 256), 256, 0, st>>>(g->off, rank.p, ub, lb, le, n, ubase, lbase); note_launch();
+  k_relabel_keys<<<grid_for(m, 256), 256, 0, st>>>(eu, ev, by_v.p, m, rank.p, ubase, lbase, nb, keys.p); note_launch();
+  by_v.release();
+  MCE_TRY(radix_sort_u64(keys.p, tmp.p, m2, nb, 2 * nb, st));
+  tmp.release();
+  MCE_CUDA_TRY(cudaMallocAsync(&g->adj, std::max<uint64_t>(m2, 1) * sizeof(uint32_t), st));
   DevBuf<uint32_t> upflag, uppos;
   MCE_TRY(upflag.alloc(m2 + 1, st));
   MCE_TRY(uppos.alloc(m2 + 1, st));
@@ -658,27 +756,22 @@ mce_status build_from_csr(uint64_t n, const uint32_t *off_d, const uint32_t *adj
   MCE_CUDA_TRY(cudaMemcpyAsync(&m2, off_d + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   MCE_CUDA_TRY(cudaStreamSynchronize(st));
   const uint64_t m = m2 / 2;
-  // edges (r < c) and degrees from the CSR
-  DevBuf<uint32_t> deg, eu, ev, labels0;
-  MCE_TRY(deg.alloc(n + 1, st));
+  // edges (r < c) from the CSR
+  DevBuf<uint32_t> eu, ev, labels0;
   MCE_TRY(labels0.alloc(n, st));
   if (labels_d)
     MCE_CUDA_TRY(cudaMemcpyAsync(labels0.p, labels_d, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
   else
     k_iota<<<grid_for(n, 256), 256, 0, st>>>(labels0.p, n); note_launch();
-  MCE_TRY(csr_to_edges(n, off_d, adj_d, m, deg.p, &eu.p, &ev.p, st));
+  MCE_TRY(csr_to_edges(n, off_d, adj_d, m, &eu.p, &ev.p, st));
   eu.st = ev.st = st;
-  MCE_TRY(finish_graph((uint32_t)n, m, eu.p, ev.p, deg.p, labels0.p,
+  MCE_TRY(finish_graph((uint32_t)n, m, eu.p, ev.p, labels0.p,
                        already_ordered ? MCE_ORDER_UNCHANGED : order_kind, spin_limit, st, g));
   if (already_ordered && degeneracy_hint) g->degeneracy = degeneracy_hint;
   return MCE_OK;
 }
 
 namespace {
-__global__ void k_degrees_from_off(const uint32_t *off, uint64_t n, uint32_t *deg) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    deg[i] = off[i + 1] - off[i];
-}
 __global__ void k_upper_flags(const uint32_t *off, const uint32_t *adj, uint64_t n, uint32_t *flag) {
   // one warp per row
   const uint32_t lane = lane_id();
@@ -699,9 +792,8 @@ __global__ void k_upper_edges(const uint32_t *off, const uint32_t *adj, uint64_t
 }
 }  // namespace
 
-mce_status csr_to_edges(uint64_t n, const uint32_t *off, const uint32_t *adj, uint64_t m, uint32_t *deg,
-                        uint32_t **eu, uint32_t **ev, cudaStream_t st) {
-  k_degrees_from_off<<<grid_for(n, 256), 256, 0, st>>>(off, n, deg); note_launch();
+mce_status csr_to_edges(uint64_t n, const uint32_t *off, const uint32_t *adj, uint64_t m, uint32_t **eu,
+                        uint32_t **ev, cudaStream_t st) {
   DevBuf<uint32_t> flag, pos;
   MCE_TRY(flag.alloc(2 * m + 1, st));
   MCE_TRY(pos.alloc(2 * m + 1, st));
