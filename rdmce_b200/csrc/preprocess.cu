@@ -144,29 +144,41 @@ __global__ void k_iota(uint32_t *a, uint64_t n) {
 // (edges of the ordered CSR) are stable from run to run; the reference's
 // sequential queue (graph.cc:289-304) orders vertices inside a round
 // differently, which changes neither the degeneracy nor the clique set.
-// A skewed graph's core peels in hundreds of levels of a few rounds each, with
-// little work in most: the time is barriers and dependent L2 accesses.  So
+// A skewed graph's core peels in hundreds of rounds with little work in most:
+// the time is a round's chain of dependent L2 accesses and its barrier.  So
 // counters are never reused (one per round and per level, cleared up front),
 // which leaves one barrier a scan and one a round; the barrier is one counter
-// that 148 blocks add to; and a warp keeps four neighbours in flight.
-// Measured (B200): R-MAT 20 (192 levels, 622 rounds) 5.3 -> 4.4 ms.
+// that 148 blocks add to, with one fence a block; a frontier entry is the
+// vertex's adjacency range, read when it is claimed; a warp keeps four
+// neighbours in flight; and small rounds decrement a neighbour without asking
+// first whether it is gone: a vertex removed at level k' <= k never has
+// residual degree k + 1 again.
+// Measured (B200): R-MAT 20 (192 levels, 622 rounds) 5.3 -> 4.1 ms, the core below
+// included.
 struct PeelCtl {
   uint32_t arrived;     // barrier arrivals so far
   uint32_t degeneracy;
   uint32_t rounds;
   uint32_t levels;
   uint32_t error;       // 1: level bound exceeded (cannot happen on a consistent CSR); 2: a barrier wait ran out
+  // where the grid stopped, for the core kernel: nrem vertices left (0: none)
+  // in list `list` (0: A, 1: B), level and round counts, next k
+  uint32_t nrem, list, lev, r, k;
 };
+// The rest of a graph is peeled by one block once it fits that block's shared
+// memory and is worth few enough neighbour visits.
+constexpr uint32_t kCoreVertices = 16384, kCoreEntries = 3u << 20;
 constexpr uint32_t kPeelThreads = 512;
+constexpr uint32_t kPeelAsk = 256;  // frontiers from this size on skip removed neighbours (atomics bound them)
 
 // One barrier of the whole grid (all blocks are resident); false when the wait
 // ran out.
 __device__ __forceinline__ bool grid_barrier(PeelCtl *ctl, uint32_t *target, uint64_t spin_limit) {
   __shared__ uint32_t ok;
   *target += gridDim.x;
-  __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
+    __threadfence();  // the block's writes, ordered before this by the barrier above
     atomicAdd(&ctl->arrived, 1u);
     uint32_t seen = 0;
     uint64_t n = 0;
@@ -175,25 +187,27 @@ __device__ __forceinline__ bool grid_barrier(PeelCtl *ctl, uint32_t *target, uin
     } while (seen < *target && ++n < spin_limit);
     ok = seen >= *target;
     if (!ok) atomicExch(&ctl->error, 2u);
-    __threadfence();
   }
   __syncthreads();
   return ok != 0;
 }
 
-// fcnt[r]: vertices claimed into round r; rcnt[l], rmin[l]: survivors of level
-// l's scan and their smallest residual degree.
+// fcnt[r]: vertices claimed into round r; rcnt[l], rmin[l], rsum[l]: survivors
+// of level l's scan, their smallest residual degree and the sum of them.
 __global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const uint32_t *off, const uint32_t *adj,
                                                               int *deg, uint32_t *state, uint32_t *remA,
-                                                              uint32_t *remB, uint32_t *frA, uint32_t *frB,
+                                                              uint32_t *remB, uint2 *frA, uint2 *frB,
                                                               PeelCtl *ctl, uint32_t *fcnt, uint32_t *rcnt,
-                                                              uint32_t *rmin, uint32_t max_levels,
+                                                              uint32_t *rmin, unsigned long long *rsum,
+                                                              uint32_t max_levels,
                                                               uint64_t spin_limit) {
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
-  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint64_t gwarp = tid >> 5, nwarps = nthreads >> 5;
   const bool leader = tid == 0;
+  __shared__ uint32_t s_at[2][kPeelThreads / 32], s_min[kPeelThreads / 32];
+  __shared__ unsigned long long s_sum[kPeelThreads / 32];
   uint32_t target = 0;
   uint32_t k = 0, degen = 0, lev = 0, r = 0, removed = 0, nrem = n;
   uint32_t *rem_cur = remA, *rem_nxt = remB;
@@ -202,14 +216,25 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const 
       if (leader) atomicExch(&ctl->error, 1u);
       break;  // uniform: every thread sees the same lev
     }
-    uint32_t *fr = (r & 1) ? frB : frA;
+    // the sum is from before the last level's rounds, so at least the true one
+    if (lev && nrem <= kCoreVertices && __ldcg(&rsum[lev - 1]) <= kCoreEntries) {
+      if (leader) {
+        ctl->nrem = nrem;
+        ctl->list = rem_cur == remB;
+        ctl->lev = lev;
+        ctl->r = r;
+        ctl->k = k;
+      }
+      break;
+    }
+    uint2 *fr = (r & 1) ? frB : frA;
     // scan: claim residual degree <= k into F_r, keep the rest
     uint32_t local_min = 0xffffffffu;
-    // warp-uniform trip count; one atomic per warp and list (every survivor
-    // is appended at every level, so per-thread atomics on one counter would
-    // serialise)
-    for (uint64_t base = tid - lane; base < nrem; base += nthreads) {
-      const uint64_t i = base + lane;
+    unsigned long long local_sum = 0;
+    // block-uniform trip count; one atomic a block and list (every survivor is
+    // appended at every level, and atomics on one counter serialise)
+    for (uint64_t base = (uint64_t)blockIdx.x * kPeelThreads; base < nrem; base += nthreads) {
+      const uint64_t i = base + threadIdx.x;
       uint32_t v = 0;
       int d = 0;
       bool claim = false, keep = false;
@@ -222,23 +247,50 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const 
         }
       }
       const uint32_t cm = __ballot_sync(kFull, claim), km = __ballot_sync(kFull, keep);
-      uint32_t cb = 0, kb = 0;
       if (lane == 0) {
-        if (cm) cb = atomicAdd(&fcnt[r], (uint32_t)__popc(cm));
-        if (km) kb = atomicAdd(&rcnt[lev], (uint32_t)__popc(km));
+        s_at[0][wid] = __popc(cm);
+        s_at[1][wid] = __popc(km);
       }
-      cb = __shfl_sync(kFull, cb, 0);
-      kb = __shfl_sync(kFull, kb, 0);
+      __syncthreads();
+      if (wid < 2) {  // warp 0: claims, warp 1: survivors
+        const uint32_t c = lane < kPeelThreads / 32 ? s_at[wid][lane] : 0;
+        uint32_t incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(kFull, incl, o);
+          if (lane >= o) incl += y;
+        }
+        uint32_t at = 0;
+        if (lane == 31 && incl) at = atomicAdd(wid ? &rcnt[lev] : &fcnt[r], incl);
+        at = __shfl_sync(kFull, at, 31);
+        if (lane < kPeelThreads / 32) s_at[wid][lane] = at + incl - c;
+      }
+      __syncthreads();
       if (claim) {
         state[v] = r + 1;
-        fr[cb + __popc(cm & lanemask_lt())] = v;
+        fr[s_at[0][wid] + __popc(cm & lanemask_lt())] = make_uint2(off[v], off[v + 1]);
       } else if (keep) {
-        rem_nxt[kb + __popc(km & lanemask_lt())] = v;
+        rem_nxt[s_at[1][wid] + __popc(km & lanemask_lt())] = v;
         local_min = min(local_min, (uint32_t)d);
+        local_sum += (uint32_t)d;
       }
+      __syncthreads();
     }
     local_min = __reduce_min_sync(kFull, local_min);
-    if (lane == 0 && local_min != 0xffffffffu) atomicMin(&rmin[lev], local_min);
+    local_sum = warp_sum_u64(local_sum);
+    if (lane == 0) {
+      s_min[wid] = local_min;
+      s_sum[wid] = local_sum;
+    }
+    __syncthreads();
+    if (wid == 0) {
+      local_min = __reduce_min_sync(kFull, lane < kPeelThreads / 32 ? s_min[lane] : 0xffffffffu);
+      local_sum = warp_sum_u64(lane < kPeelThreads / 32 ? s_sum[lane] : 0);
+      if (lane == 0 && local_min != 0xffffffffu) {
+        atomicMin(&rmin[lev], local_min);
+        atomicAdd(&rsum[lev], local_sum);
+      }
+    }
     if (!grid_barrier(ctl, &target, spin_limit)) return;
     uint32_t level_claims = 0;
     for (;;) {
@@ -246,18 +298,18 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const 
       if (nf == 0) break;
       level_claims += nf;
       removed += nf;
-      const uint32_t *cur = (r & 1) ? frB : frA;
-      uint32_t *nxt = (r & 1) ? frA : frB;
+      const uint2 *cur = (r & 1) ? frB : frA;
+      uint2 *nxt = (r & 1) ? frA : frB;
       // Each frontier vertex's adjacency is shared by `per` warps (all the
       // grid's warps split evenly when the frontier is small: the dense
       // cores' hubs hold tens of thousands of neighbours each).
       const uint64_t per = nf < nwarps ? nwarps / nf : 1;
       for (uint64_t i = gwarp / per; i < nf; i += nwarps / per) {
-        const uint32_t v = __ldcg(cur + i);
-        const uint32_t e1 = off[v + 1];
+        const uint2 range = __ldcg(cur + i);
+        const uint32_t e1 = range.y;
         const uint32_t part = (uint32_t)(gwarp % per);
         const uint64_t step = 32ULL * per;
-        for (uint64_t e = (uint64_t)off[v] + 32ULL * part + lane; e < e1; e += 4 * step) {
+        for (uint64_t e = (uint64_t)range.x + 32ULL * part + lane; e < e1; e += 4 * step) {
           uint32_t u[4];
           bool open[4];
 #pragma unroll
@@ -265,8 +317,10 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const 
             open[j] = e + j * step < e1;
             u[j] = open[j] ? adj[e + j * step] : 0;
           }
+          if (nf >= kPeelAsk) {
 #pragma unroll
-          for (int j = 0; j < 4; j++) open[j] = open[j] && !__ldcg(state + u[j]);
+            for (int j = 0; j < 4; j++) open[j] = open[j] && !__ldcg(state + u[j]);
+          }
           int was[4];
 #pragma unroll
           for (int j = 0; j < 4; j++) was[j] = open[j] ? atomicSub(&deg[u[j]], 1) : 0;
@@ -274,7 +328,8 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const 
           for (int j = 0; j < 4; j++)
             if (open[j] && was[j] == (int)k + 1) {  // one decrement alone sees k + 1: it claims the vertex
               state[u[j]] = r + 2;
-              nxt[atomicAdd(&fcnt[r + 1], 1u)] = u[j];
+              const uint2 next = make_uint2(off[u[j]], off[u[j] + 1]);
+              nxt[atomicAdd(&fcnt[r + 1], 1u)] = next;
             }
         }
       }
@@ -302,6 +357,173 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const 
     // writes are not read any more.
   }
   if (leader) {
+    ctl->degeneracy = degen;
+    ctl->rounds = r;
+    ctl->levels = lev;
+  }
+}
+
+// The vertices that are left: their numbers in the list, and their residual
+// degrees, which are their numbers of neighbours left.  One of the list's
+// vertices may have been claimed in the level's last rounds: degree 0 here.
+__global__ void k_core_ids(const PeelCtl *ctl, const uint32_t *remA, const uint32_t *remB, const uint32_t *state,
+                           const int *deg, uint32_t *id, uint32_t *cdeg) {
+  const uint32_t *rem = ctl->list ? remB : remA;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kCoreVertices; i += gridDim.x * blockDim.x) {
+    uint32_t d = 0;
+    if (i < ctl->nrem) {
+      const uint32_t v = rem[i];
+      id[v] = i;
+      if (!state[v]) d = (uint32_t)deg[v];
+    }
+    cdeg[i] = d;
+  }
+}
+
+// their adjacency among themselves (in any order), one block a vertex: a hub
+// still has its whole list
+__global__ void __launch_bounds__(256) k_core_fill(const PeelCtl *ctl, const uint32_t *remA, const uint32_t *remB,
+                                                   const uint32_t *off, const uint32_t *adj, const uint32_t *state,
+                                                   const uint32_t *id, const uint32_t *coff, uint16_t *cadj) {
+  __shared__ uint32_t s_at;
+  const uint32_t *rem = ctl->list ? remB : remA;
+  const uint32_t lane = threadIdx.x & 31, nrem = ctl->nrem;
+  for (uint32_t i = blockIdx.x; i < nrem; i += gridDim.x) {
+    const uint32_t v = rem[i];
+    if (state[v]) continue;
+    if (threadIdx.x == 0) s_at = coff[i];
+    __syncthreads();
+    const uint32_t e1 = off[v + 1];
+    for (uint64_t base = (uint64_t)off[v] + threadIdx.x - lane; base < e1; base += 4 * 256) {
+      uint32_t u[4];
+      bool left[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        left[j] = base + j * 256 + lane < e1;
+        u[j] = left[j] ? adj[base + j * 256 + lane] : 0;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) left[j] = left[j] && !state[u[j]];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const uint32_t bal = __ballot_sync(kFull, left[j]);
+        uint32_t at = 0;
+        if (lane == 0 && bal) at = atomicAdd(&s_at, (uint32_t)__popc(bal));
+        at = __shfl_sync(kFull, at, 0);
+        if (left[j]) cadj[at + __popc(bal & lanemask_lt())] = (uint16_t)id[u[j]];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The remaining rounds, in one block: residual degrees (negative once removed),
+// list offsets and frontiers in shared memory, so that a round waits on one
+// global load, the neighbours.  A round of the whole grid costs about 5 us,
+// nearly all of it dependent L2 accesses and the barrier; here it costs 1 to
+// 2 us.  Same rounds, so same order.
+// Measured (B200), whole build: R-MAT 14 (all of it here) 1.65 -> 1.38 ms,
+// R-MAT 17 3.1 -> 2.9 ms; 6 M entries instead of 3 M cost R-MAT 20 0.5 ms.
+constexpr uint32_t kCoreThreads = 1024;
+constexpr size_t kCoreSmem = (kCoreVertices + 4) * (2 * sizeof(int) + 2 * sizeof(uint16_t));
+
+__global__ void __launch_bounds__(kCoreThreads) k_peel_core(PeelCtl *ctl, const uint32_t *remA, const uint32_t *remB,
+                                                            uint32_t *state, const uint32_t *cdeg,
+                                                            const uint32_t *coff, const uint16_t *cadj,
+                                                            uint32_t *cround) {
+  extern __shared__ int sdeg[];
+  uint32_t *soff = (uint32_t *)(sdeg + kCoreVertices);  // n + 1
+  uint16_t *fr[2] = {(uint16_t *)(soff + kCoreVertices + 4), (uint16_t *)(soff + kCoreVertices + 4) + kCoreVertices};
+  __shared__ uint32_t cnt[3];  // frontier sizes, by round mod 3
+  __shared__ uint32_t s_min;
+  const uint32_t n = ctl->nrem;
+  if (n == 0) return;
+  const uint32_t *rem = ctl->list ? remB : remA;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarps = kCoreThreads / 32;
+  constexpr int kGone = -(1 << 30);
+  uint32_t gone = 0;
+  for (uint32_t i = tid; i < n; i += kCoreThreads) {
+    const bool left = !state[rem[i]];
+    sdeg[i] = left ? (int)cdeg[i] : kGone;
+    cround[i] = 0;
+    gone += !left;
+  }
+  for (uint32_t i = tid; i <= n; i += kCoreThreads) soff[i] = coff[i];
+  if (tid < 3) cnt[tid] = 0;
+  __syncthreads();
+  if (gone) atomicAdd(&cnt[0], gone);
+  __syncthreads();
+  uint32_t left = n - cnt[0];
+  uint32_t k = ctl->k, r = ctl->r, lev = ctl->lev, degen = ctl->degeneracy;
+  __syncthreads();
+  if (tid == 0) cnt[0] = 0;
+  while (left) {
+    if (tid == 0) s_min = 0xffffffffu;
+    __syncthreads();
+    // scan: claim residual degree <= k
+    uint32_t least = 0xffffffffu;
+    for (uint32_t base = tid - lane; base < n; base += kCoreThreads) {
+      const uint32_t i = base + lane;
+      const int d = i < n ? sdeg[i] : kGone;
+      const bool claim = d >= 0 && d <= (int)k;
+      if (d > (int)k) least = min(least, (uint32_t)d);
+      const uint32_t bal = __ballot_sync(kFull, claim);
+      uint32_t at = 0;
+      if (lane == 0 && bal) at = atomicAdd(&cnt[r % 3], (uint32_t)__popc(bal));
+      at = __shfl_sync(kFull, at, 0);
+      if (claim) {
+        sdeg[i] = kGone;
+        cround[i] = r + 1;
+        fr[r & 1][at + __popc(bal & lanemask_lt())] = (uint16_t)i;
+      }
+    }
+    least = __reduce_min_sync(kFull, least);
+    if (lane == 0 && least != 0xffffffffu) atomicMin(&s_min, least);
+    __syncthreads();
+    uint32_t claims = 0;
+    for (;;) {
+      const uint32_t nf = cnt[r % 3];
+      if (nf == 0) break;
+      claims += nf;
+      left -= nf;
+      if (tid == 0) cnt[(r + 2) % 3] = 0;  // last read in round r - 1
+      const uint16_t *cur = fr[r & 1];
+      uint16_t *nxt = fr[(r + 1) & 1];
+      const uint32_t per = nf < nwarps ? nwarps / nf : 1;
+      for (uint32_t i = wid / per; i < nf; i += nwarps / per) {
+        const uint32_t x = cur[i], e1 = soff[x + 1], step = 32 * per;
+        for (uint32_t e = soff[x] + 32 * (wid % per) + lane; e < e1; e += 4 * step) {
+          uint32_t u[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) u[j] = e + j * step < e1 ? cadj[e + j * step] : 0xffffffffu;
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            if (u[j] == 0xffffffffu || atomicSub(&sdeg[u[j]], 1) != (int)k + 1) continue;
+            sdeg[u[j]] = kGone;
+            cround[u[j]] = r + 2;
+            nxt[atomicAdd(&cnt[(r + 1) % 3], 1u)] = (uint16_t)u[j];
+          }
+        }
+      }
+      __syncthreads();
+      r++;
+    }
+    // as on the grid: an empty round separates the levels
+    r++;
+    if (claims) {
+      degen = k;
+      k++;
+    } else {
+      k = max(k + 1, s_min);
+    }
+    lev++;
+    __syncthreads();
+    if (tid < 3) cnt[tid] = 0;
+  }
+  __syncthreads();
+  for (uint32_t i = tid; i < n; i += kCoreThreads)
+    if (cround[i]) state[rem[i]] = cround[i];
+  if (tid == 0) {
     ctl->degeneracy = degen;
     ctl->rounds = r;
     ctl->levels = lev;
@@ -423,9 +645,10 @@ mce_status read_scalar(const T *d, T *h, cudaStream_t st) {
 
 // k-core peeling over an unsorted symmetric CSR; fills order[] (position -> vertex)
 mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint32_t *deg0, uint32_t max_degree,
-                uint32_t *order, uint32_t *degeneracy, uint64_t spin_limit, cudaStream_t st) {
+                uint64_t entries, uint32_t *order, uint32_t *degeneracy, uint64_t spin_limit, cudaStream_t st) {
   DevBuf<int> deg;
-  DevBuf<uint32_t> state, remA, remB, frA, frB;
+  DevBuf<uint32_t> state, remA, remB;
+  DevBuf<uint2> frA, frB;
   DevBuf<PeelCtl> ctl;
   MCE_TRY(deg.alloc(n, st));
   MCE_TRY(state.alloc(n, st));
@@ -440,32 +663,58 @@ mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint
   // one counter a round (every round but the last of a level claims a vertex)
   // and two a level
   const uint64_t max_levels = (uint64_t)max_degree + 2, max_rounds = (uint64_t)n + max_levels + 4;
+  const bool core_only = n <= kCoreVertices && entries <= kCoreEntries;
   DevBuf<uint32_t> counters;
-  MCE_TRY(counters.alloc(max_rounds + 2 * (max_levels + 2), st));
+  DevBuf<unsigned long long> sums;
+  if (!core_only) {
+    MCE_TRY(counters.alloc(max_rounds + 2 * (max_levels + 2), st));
+    MCE_TRY(sums.alloc(max_levels + 2, st));
+  }
   uint32_t *fcnt = counters.p, *rcnt = fcnt + max_rounds, *rmin = rcnt + max_levels + 2;
-  MCE_CUDA_TRY(cudaMemsetAsync(fcnt, 0, (max_rounds + max_levels + 2) * sizeof(uint32_t), st));
-  MCE_CUDA_TRY(cudaMemsetAsync(rmin, 0xff, (max_levels + 2) * sizeof(uint32_t), st));
-  MCE_CUDA_TRY(cudaMemsetAsync(ctl.p, 0, sizeof(PeelCtl), st));
-  // the control block is read through ordinary host memory: pinning it for
-  // each build (and unpinning, which synchronises the device) would stall
-  // other streams' work, e.g. concurrently served requests
+  unsigned long long *rsum = sums.p;
+  // the control block goes through ordinary host memory: pinning it for each
+  // build (and unpinning, which synchronises the device) would stall other
+  // streams' work, e.g. concurrently served requests
   PeelCtl h{};
   PeelCtl *hc = &h;
-  int dev = 0, sms = 0, per_sm = 0;
-  MCE_CUDA_TRY(cudaGetDevice(&dev));
-  MCE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  MCE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel_rounds, kPeelThreads, 0));
-  if (per_sm < 1) return MCE_ERR_INTERNAL;
-  // a cooperative launch: every block is resident, so the barrier is sound
-  const uint32_t blocks = (uint32_t)sms;
-  uint32_t nn = n, maxl = (uint32_t)max_levels;
-  int *degp = deg.p;
-  uint32_t *statep = state.p, *ra = remA.p, *rb = remB.p, *fa = frA.p, *fb = frB.p;
-  PeelCtl *cp = ctl.p;
-  void *args[] = {&nn, (void *)&off, (void *)&adj, &degp, &statep, &ra, &rb, &fa, &fb, &cp, &fcnt, &rcnt, &rmin, &maxl,
-                  &spin_limit};
-  MCE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_peel_rounds, dim3(blocks), dim3(kPeelThreads), args, 0, st));
-  note_launch();
+  if (core_only) h.nrem = n;
+  MCE_CUDA_TRY(cudaMemcpyAsync(ctl.p, hc, sizeof(PeelCtl), cudaMemcpyHostToDevice, st));
+  if (!core_only) {
+    MCE_CUDA_TRY(cudaMemsetAsync(fcnt, 0, (max_rounds + max_levels + 2) * sizeof(uint32_t), st));
+    MCE_CUDA_TRY(cudaMemsetAsync(rmin, 0xff, (max_levels + 2) * sizeof(uint32_t), st));
+    MCE_CUDA_TRY(cudaMemsetAsync(rsum, 0, (max_levels + 2) * sizeof(unsigned long long), st));
+    int dev = 0, sms = 0, per_sm = 0;
+    MCE_CUDA_TRY(cudaGetDevice(&dev));
+    MCE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MCE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_peel_rounds, kPeelThreads, 0));
+    if (per_sm < 1) return MCE_ERR_INTERNAL;
+    // a cooperative launch: every block is resident, so the barrier is sound
+    const uint32_t blocks = (uint32_t)sms;
+    uint32_t nn = n, maxl = (uint32_t)max_levels;
+    int *degp = deg.p;
+    uint32_t *statep = state.p, *ra = remA.p, *rb = remB.p;
+    uint2 *fa = frA.p, *fb = frB.p;
+    PeelCtl *cp = ctl.p;
+    void *args[] = {&nn, (void *)&off, (void *)&adj, &degp, &statep, &ra, &rb, &fa, &fb, &cp, &fcnt, &rcnt, &rmin, &rsum,
+                    &maxl, &spin_limit};
+    MCE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_peel_rounds, dim3(blocks), dim3(kPeelThreads), args, 0, st));
+    note_launch();
+  }
+  {
+    DevBuf<uint32_t> core;  // residual degrees and offsets of the vertices left
+    DevBuf<uint16_t> cadj;
+    MCE_TRY(core.alloc(3 * kCoreVertices + 1, st));
+    MCE_TRY(cadj.alloc(std::min<uint64_t>(entries, kCoreEntries), st));
+    uint32_t *cdeg = core.p, *coff = cdeg + kCoreVertices, *cround = coff + kCoreVertices + 1;
+    uint32_t *id = (uint32_t *)frA.p;
+    k_core_ids<<<kCoreVertices / 256, 256, 0, st>>>(ctl.p, remA.p, remB.p, state.p, deg.p, id, cdeg); note_launch();
+    MCE_TRY(scan_exclusive_u32(cdeg, coff, kCoreVertices, coff + kCoreVertices, st));
+    k_core_fill<<<grid_for(std::min(n, kCoreVertices), 1, 148 * 8), 256, 0, st>>>(ctl.p, remA.p, remB.p, off, adj, state.p, id, coff, cadj.p); note_launch();
+    MCE_CUDA_TRY(cudaFuncSetAttribute(k_peel_core, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoreSmem));
+    k_peel_core<<<1, kCoreThreads, kCoreSmem, st>>>(ctl.p, remA.p, remB.p, state.p, cdeg, coff, cadj.p,
+                                                      cround); note_launch();
+    MCE_CUDA_TRY(cudaGetLastError());
+  }
   MCE_CUDA_TRY(cudaMemcpyAsync(hc, ctl.p, sizeof(PeelCtl), cudaMemcpyDeviceToHost, st));
   MCE_CUDA_TRY(cudaStreamSynchronize(st));
   if (h.error) return h.error == 2 ? MCE_ERR_TIMEOUT : MCE_ERR_INTERNAL;
@@ -696,7 +945,7 @@ mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32
     MCE_TRY(scan_exclusive_u32(deg.p, off0.p, n, off0.p + n, st));
     k_run_bases<<<grid_for(n, 256), 256, 0, st>>>(off0.p, nullptr, ub, lb, le, n, ubase, lbase); note_launch();
     k_fill_adj<<<grid_for(m, 256), 256, 0, st>>>(eu, ev, by_v.p, m, nb, ubase, lbase, adj0.p); note_launch();
-    MCE_TRY(peel(n, off0.p, adj0.p, deg.p, g->max_degree, order.p, &g->degeneracy, spin_limit, st));
+    MCE_TRY(peel(n, off0.p, adj0.p, deg.p, g->max_degree, m2, order.p, &g->degeneracy, spin_limit, st));
   } else if ((order_kind == MCE_ORDER_DEGREE_ASC || order_kind == MCE_ORDER_DEGREE_DESC) && n > 0) {
     DevBuf<uint64_t> dk, dt;
     MCE_TRY(dk.alloc(n, st));
