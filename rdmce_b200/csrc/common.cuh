@@ -119,7 +119,7 @@ mce_status reduce_max_u32(const uint32_t *in, uint64_t n, uint32_t *d_out, cudaS
 // on demand and kept for reuse (the role of the reference's BufferManager,
 // include/context_gpu.cuh:4-32, without its worst-case sizing).
 struct Scratch {
-  static constexpr int kSlots = 9;
+  static constexpr int kSlots = 10;
   int device = 0;
   // set: buffers are allocated and freed stream-ordered on this stream (no
   // device-wide synchronisation when one grows), for an owner whose work

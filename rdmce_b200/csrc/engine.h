@@ -144,7 +144,9 @@ struct EnumParams {
   const uint64_t *root_list;             // list mode: root ids (else the range [rb, re))
   uint64_t n_list;                       // entries in root_list
   int vertex_pass;                       // work items are the vertices of the range, not its roots
-  uint64_t single_items;                 // vertex pass: claims of one vertex; later claims take kVertexChunk
+  uint32_t *vert_list;                   // vertex pass: after the last single_items vertices, those to take (null: all)
+  uint64_t single_items;
+  unsigned int *vert_n;                  // how many
   uint32_t *edge_out;                    // vertex pass: roots left to the edge pass
   unsigned int *edge_n;                  // how many
   const uint32_t *edge_list;             // edge pass: those roots (edge_n of them)
@@ -238,6 +240,8 @@ MCE_DECLARE_ENUM_BUILD(3)
 MCE_DECLARE_ENUM_BUILD(4)
 MCE_DECLARE_ENUM_BUILD(5)
 #undef MCE_DECLARE_ENUM_BUILD
+// the vertices of few later neighbours (tiny.cu); lists the others in P.vert_list
+mce_status launch_tiny(const EnumParams &P, uint32_t sms, cudaStream_t st);
 mce_status probe_int_peak(int device, double *word_ops_per_s);
 
 }  // namespace mce

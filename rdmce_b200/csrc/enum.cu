@@ -78,9 +78,10 @@ constexpr uint32_t kLocalRec = 2048;      // per-warp local task record (64-bit-
 // with fewer, larger tasks, once nested tiers expose their outer levels first.
 constexpr uint32_t kRegShareBound = 24;
 constexpr uint32_t kShareMin = 128, kShareMax = 8192;
-// Vertex pass: the first claims (the core's vertices) take one vertex, later
-// ones kVertexChunk, since a claim costs as much as a small vertex's work.
-constexpr uint32_t kVertexChunk = 8, kVertexSingles = 8;  // single claims: kVertexSingles a warp
+// A graph with more vertices than this for each warp has the others' small
+// vertices decided up front, 32 to a warp (tiny.cu); the late-peeled ones, up
+// to this many, are items in order either way.
+constexpr uint32_t kVertexSingles = 8;
 // 32-bit-tier nodes with up to this many candidates are decided in one step,
 // at 2^(n - 5) groups of about 12 instructions each (t0_small_sets).
 #ifndef MCE_SMALL_P
@@ -2492,10 +2493,12 @@ __device__ bool solve_root(const Ctx &c, uint64_t r) {
 }
 
 // Vertices solved whole.  Up to kVertexCols later neighbours and kVertexDegree
-// neighbours a vertex's ego network is built once and searched with a pivot;
+// neighbours (a hub's members are many warps' work: Chung-Lu 10^6 6.4 ms with
+// up to 16384, 5.6 with 4096, 5.8 with 2048, where full R-MAT 14 loses 10 %) a
+// vertex's ego network is built once and searched with a pivot;
 // from 65 later neighbours on (the general tier) only where at most
 // kVertexBranches of them, and at most a quarter, are left to branch on.
-constexpr uint32_t kVertexCols = 256, kVertexDegree = 16384, kVertexBranches = 16;
+constexpr uint32_t kVertexCols = 256, kVertexDegree = 4096, kVertexBranches = 16;
 
 // Vertex item k of the vertex pass: the cliques whose first vertex (in the
 // order) is v.  An edge root (v, w) builds its own ego network out of the
@@ -2509,7 +2512,8 @@ constexpr uint32_t kVertexCols = 256, kVertexDegree = 16384, kVertexBranches = 1
 __device__ __noinline__ uint32_t run_vertex(Ctx c, uint64_t k) {
   const EnumParams &P = *c.P;
   const DevGraph &g = P.g;
-  const uint32_t v = g.n - 1 - (uint32_t)k;  // late-peeled vertices first
+  // late-peeled vertices first: they are the heavy ones
+  const uint32_t v = P.vert_list && k >= P.single_items ? P.vert_list[k - P.single_items] : g.n - 1 - (uint32_t)k;
   const uint32_t r0 = g.root_off[v], r1 = g.root_off[v + 1];
   const uint32_t lo = (uint32_t)max((uint64_t)r0, P.rb), hi = (uint32_t)min((uint64_t)r1, P.re);
   if (lo >= hi) return 0;
@@ -2748,7 +2752,7 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
   c.ta = (T1Area *)(c.slab + c.slab_bytes - kTail);
   c.sharing = P.sharing != 0;
   const uint64_t total = P.heavy_list    ? P.n_heavy
-                         : P.vertex_pass ? P.single_items + (P.g.n - P.single_items + kVertexChunk - 1) / kVertexChunk
+                         : P.vertex_pass ? (P.vert_list ? P.single_items + *P.vert_n : P.g.n)
                          : P.edge_list   ? *P.edge_n
                          : P.root_list   ? P.n_list
                                          : P.re - P.rb;
@@ -2779,12 +2783,7 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
     k = __shfl_sync(kFull, k, 0);
     if (k >= total) break;
     if (P.vertex_pass) {
-      uint64_t v = k, e = k + 1;
-      if (k >= P.single_items) {
-        v = P.single_items + (k - P.single_items) * kVertexChunk;
-        e = min(v + kVertexChunk, (uint64_t)P.g.n);
-      }
-      for (; v < e; v++) nroots += run_vertex(c, v);
+      nroots += run_vertex(c, k);
       continue;
     }
     nroots++;
@@ -2831,7 +2830,7 @@ struct EnumCtl {
   alignas(128) unsigned long long heavy_need, stat_roots, stat_tasks, stat_nodes, stat_wops, stat_bbytes;
   unsigned long long stat_cycles[kCycPhases];
   unsigned long long stat_max_item[2];
-  unsigned int heavy_n, error, edge_n;
+  unsigned int heavy_n, error, edge_n, vert_n;
 };
 
 // free ring full of every block, ready ring empty, counters reset
@@ -2996,7 +2995,12 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
     if (!P.edge_out) return s;
     P.edge_n = &ctl->edge_n;
     P.vertex_pass = 1;
-    P.single_items = std::min<uint64_t>(g.n, kVertexSingles * nwarps);
+    if (g.n > kVertexSingles * nwarps) {
+      P.vert_list = (uint32_t *)scr->get(9, (uint64_t)g.n * 4, &s);
+      if (!P.vert_list) return s;
+      P.vert_n = &ctl->vert_n;
+      P.single_items = kVertexSingles * nwarps;
+    }
   }
   P.heavy_out = heavy;
   P.heavy_cap = (uint32_t)heavy_cap;
@@ -3016,6 +3020,7 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
 mce_status MCE_ENUM_FN(enum_launch)(const EnumPlan &plan, cudaStream_t st) {
   MCE_TRY(reset_ctl(plan, st));
   if (plan.nwork) {
+    if (plan.params.vert_list) MCE_TRY(launch_tiny(plan.params, plan.sms, st));
     k_enumerate<<<plan.blocks, plan.threads, plan.smem, st>>>(plan.params);
     note_launch();
     if (plan.vertex_pass) {
@@ -3033,7 +3038,7 @@ mce_status MCE_ENUM_FN(enum_finish)(const EnumPlan &plan, cudaStream_t st, EnumS
   MCE_CUDA_TRY(cudaMemcpyAsync(&h, ctl, sizeof(EnumCtl), cudaMemcpyDeviceToHost, st));
   MCE_CUDA_TRY(cudaStreamSynchronize(st));
   const uint64_t heavy_roots = h.heavy_n;
-  uint64_t launches = plan.nwork ? (plan.vertex_pass ? 2 : 1) : 0;
+  uint64_t launches = plan.nwork ? (plan.params.vert_list ? 3 : plan.vertex_pass ? 2 : 1) : 0;
   uint64_t roots = h.stat_roots;
   uint64_t tasks = h.stat_tasks, nodes = h.stat_nodes, wops = h.stat_wops, bbytes = h.stat_bbytes;
   uint64_t cycles[kCycPhases];
