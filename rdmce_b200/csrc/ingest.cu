@@ -40,7 +40,12 @@ namespace mce {
 namespace {
 
 constexpr uint64_t kTile = 8192;           // bytes per warp tile
-constexpr uint64_t kStageBytes = 64 << 20;  // pinned staging chunk
+// Pinned staging, two chunks of this size: pinning memory costs about 0.4 ms a
+// MiB, more than reading the file into it, so the chunks are only as large as
+// the overlap of reading and copying needs.  Measured (B200): R-MAT 17 as text
+// (27 MB) to a resident graph 28.8 -> 7.0 ms with 1 MiB instead of up to 64, R-MAT 20
+// (211 MB) 105 -> 31 ms; 9.9 and 36 ms with 2 MiB, 10.5 and 35 with 4.
+constexpr uint64_t kStageBytes = 1 << 20;
 constexpr int kWarpsPerBlock = 8;
 
 // number of '\n' bytes in a 32-bit word
