@@ -141,7 +141,9 @@ class Result:
 
     @classmethod
     def _from(cls, r: _Result) -> "Result":
-        hist = {s: int(r.hist[s]) for s in range(HIST_LEN) if r.hist[s]}
+        bins = np.ctypeslib.as_array(r.hist)  # reading 8192 ctypes items one by one takes longer than a small solve
+        sizes = np.flatnonzero(bins)
+        hist = dict(zip(sizes.tolist(), bins[sizes].tolist()))
         return cls(r.count, r.checksum, hist, r.max_size, r.degeneracy, r.max_degree, r.num_vertices,
                    r.num_edges, r.roots, r.shared_tasks, r.heavy_roots, list(r.phase_ms), r.nodes, r.word_ops,
                    r.launches, list(r.warp_cycles), list(r.max_item_cycles), r.build_bytes, r.blocks_per_sm,
@@ -457,8 +459,8 @@ class Batch:
         ms = C.c_double()
         _check(lib().mce_batch_solve(self.h, C.byref(opts) if opts else None, C.cast(res, C.c_void_p), _ptr(hist),
                                      hist_len, C.byref(ms)), "mce_batch_solve")
-        out = [{"count": r.count, "checksum": r.checksum, "max_size": r.max_size, "num_vertices": r.num_vertices,
-                "num_edges": r.num_edges} for r in res]
+        keys = [name for name, _type in _BatchResult._fields_]
+        out = [dict(zip(keys, row)) for row in np.ctypeslib.as_array(res).tolist()]
         return out, hist.reshape(self.n_graphs, hist_len), ms.value
 
     def close(self):
