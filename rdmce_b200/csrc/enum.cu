@@ -2675,7 +2675,8 @@ __device__ __noinline__ void run_root(Ctx c, uint64_t k) {
 // no work is left -- except for a task taken between the two reads, whose
 // taker then finishes everything it exposes by itself if all others have
 // left.  Exit waits for two such observations a back-off apart, which makes
-// that case rare.  Not inlined, so its loop holds only a few values: idle
+// that case rare; the block's other warps then leave with the poller (token
+// value 2), instead of each waiting for its own two.  Not inlined, so its loop holds only a few values: idle
 // polling costs no reloads of the caller's state.
 __device__ __noinline__ int idle_wait(Ctx c, unsigned int *s_poll) {
   const EnumParams &P = *c.P;
@@ -2687,7 +2688,10 @@ __device__ __noinline__ int idle_wait(Ctx c, unsigned int *s_poll) {
     if (c.lane == 0) {
       const unsigned long long ti0 = now();
       bool polled = false, seen = false;
-      if (atomicCAS(s_poll, 0u, 1u) == 0u) {
+      const unsigned int token = atomicCAS(s_poll, 0u, 1u);
+      if (token == 2u) {
+        result = -1;
+      } else if (token == 0u) {
         polled = true;
         const uint32_t act = *(volatile unsigned int *)P.active;
         __threadfence();
@@ -2704,7 +2708,7 @@ __device__ __noinline__ int idle_wait(Ctx c, unsigned int *s_poll) {
         } else {
           quiet = 0;
         }
-        atomicExch(s_poll, 0u);
+        atomicExch(s_poll, result == -1 ? 2u : 0u);
       }
       if (result == -2) {
         if (++idle_spins > P.spin_limit) {
@@ -2751,6 +2755,7 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
   c.slab_bytes = P.slab_bytes;
   c.ta = (T1Area *)(c.slab + c.slab_bytes - kTail);
   c.sharing = P.sharing != 0;
+  if (P.edge_list && !P.heavy_list && *P.edge_n == 0) return;  // the vertex pass left nothing (all blocks agree)
   const uint64_t total = P.heavy_list    ? P.n_heavy
                          : P.vertex_pass ? (P.vert_list ? P.single_items + *P.vert_n : P.g.n)
                          : P.edge_list   ? *P.edge_n
@@ -2942,14 +2947,22 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   P.nwarps = (uint32_t)nwarps;
   // slab: the largest ego network this graph can produce (p <= degeneracy,
   // rows <= max degree), capped at 4 MB per warp and by free memory
-  size_t freeb = 0, totalb = 0;
-  MCE_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
   const uint64_t kcap = std::max<uint32_t>(1, std::min(g.degeneracy, g.max_degree));
   const uint64_t dcap = std::max<uint32_t>(1, g.max_degree);
   const Layout LB = layout_for(dcap, (uint32_t)kcap, (uint32_t)(kcap + dcap), (uint32_t)((kcap + 63) / 64));
   const uint64_t bound = align8(LB.need + 3ULL * (kcap + dcap) * 4);
   const uint64_t slab_cap = cfg.slab_kib ? std::max<uint64_t>(16, cfg.slab_kib) << 10 : 4ULL << 20;
   uint64_t slab_bytes = std::max<uint64_t>(std::min<uint64_t>(bound, slab_cap), 16ULL << 10);
+  // Free memory limits what is newly allocated: asking for it costs tens of
+  // microseconds, so scratch that already holds the full sizes is used as it is.
+  const uint32_t pool_max = 1u << 14;
+  const auto block_size = [](uint64_t slab) {
+    return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(4096, align8(slab / 4)), 64 << 10);
+  };
+  size_t freeb = SIZE_MAX, totalb = 0;
+  if (scr->bytes[2] < ((slab_bytes + 255) & ~255ULL) * nwarps ||
+      scr->bytes[5] < (uint64_t)pool_max * block_size((slab_bytes + 255) & ~255ULL))
+    MCE_CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
   while (slab_bytes > (64ULL << 10) && slab_bytes * nwarps > freeb / 2) slab_bytes >>= 1;
   slab_bytes = (slab_bytes + 255) & ~255ULL;  // every warp's slab (and its T1Area) 256-byte aligned
   plan->fits_all = slab_bytes >= bound;
@@ -2965,9 +2978,8 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
     if (!heavy) return s;
   }
   // task pool: one record per block; both rings have one cell per block
-  const uint32_t block_bytes =
-      (uint32_t)std::min<uint64_t>(std::max<uint64_t>(4096, align8(slab_bytes / 4)), 64 << 10);
-  uint32_t nblocks = 1u << 14;
+  const uint32_t block_bytes = block_size(slab_bytes);
+  uint32_t nblocks = pool_max;
   while ((uint64_t)nblocks * block_bytes > (freeb / 8) && nblocks > 1024) nblocks >>= 1;
   char *pool = (char *)scr->get(5, (uint64_t)nblocks * block_bytes, &s);
   if (!pool) return s;
