@@ -2779,15 +2779,17 @@ __device__ __noinline__ void run_root(Ctx c, uint64_t k) {
 // left anywhere (or the wait's bound ran out: the error word says so).
 //
 // At most one warp per block polls the global queue at a time (the block's
-// poll token); the others sleep.  A warp counts itself busy only after it has
-// taken a task, so a failed attempt costs no atomic on the busy count.
-// Reading the busy count before the queue: a task is published before its
-// producer stops counting as busy, so "nobody busy" then "queue empty" means
-// no work is left -- except for a task taken between the two reads, whose
-// taker then finishes everything it exposes by itself if all others have
-// left.  Exit waits for two such observations a back-off apart, which makes
-// that case rare; the block's other warps then leave with the poller (token
-// value 2), instead of each waiting for its own two.  Not inlined, so its loop holds only a few values: idle
+// poll token); the others sleep.  A task is published before its producer
+// stops counting as busy, and a taker counts itself busy before it takes, so a
+// task is in the queue's count or its warp in the busy count at any time.  "No
+// work left" is nobody busy, queue empty, nobody busy: with only one look at
+// the busy count, before the queue's, a task taken between the two was missed,
+// and where one task hopped from warp to warp (the narrow top of a deep tree)
+// half of the blocks left before the work it still held came out: full R-MAT
+// 14 then ran its second half on 1600 of 3552 warps (25 ms instead of 16).
+// Exit waits for two such observations a back-off apart; the block's other
+// warps then leave with the poller (token value 2), instead of each waiting
+// for its own two.  Not inlined, so its loop holds only a few values: idle
 // polling costs no reloads of the caller's state.
 __device__ __noinline__ int idle_wait(Ctx c, unsigned int *s_poll) {
   const EnumParams &P = *c.P;
@@ -2809,15 +2811,18 @@ __device__ __noinline__ int idle_wait(Ctx c, unsigned int *s_poll) {
         if (*(volatile int *)P.ready_count > 0) {
           seen = true;
           uint32_t b = 0;
-          if (ring_pop(P.ready_slot, P.ready_seq, P.ready_head, P.ready_count, P.pool_mask, &b, P)) {
-            atomicAdd(P.active, 1u);
-            result = (int)b;
-          }
+          atomicAdd(P.active, 1u);
+          __threadfence();
+          if (ring_pop(P.ready_slot, P.ready_seq, P.ready_head, P.ready_count, P.pool_mask, &b, P)) result = (int)b;
+          else atomicSub(P.active, 1u);
           quiet = 0;
-        } else if (act == 0) {
-          if (++quiet >= 2) result = -1;
         } else {
-          quiet = 0;
+          __threadfence();
+          if (act == 0 && *(volatile unsigned int *)P.active == 0) {
+            if (++quiet >= 2) result = -1;
+          } else {
+            quiet = 0;
+          }
         }
         atomicExch(s_poll, result == -1 ? 2u : 0u);
       }
