@@ -25,11 +25,13 @@
 //     a smaller tier has its rows compressed to its own columns (parallel bit
 //     compress) and gathered, and continues there.
 //   * In the 32-bit tier R is a column mask and leaves are hashed 32 at a
-//     time, one per lane.  A node or child with at most 5 candidates is
-//     decided in one step: its maximal cliques are the cliques K of the
-//     candidates that no active row contains, and lane i tests the i-th
-//     subset.  The node loop makes no calls; to expose work it steps out
-//     and is resumed.
+//     time, one per lane.  A node or child with few candidates is decided in
+//     one step: its maximal cliques are the cliques K of the candidates that
+//     no active row contains, found on words of subsets.  To expose work the
+//     node loop steps out and is resumed.
+//   * A range of roots is taken vertex by vertex first: one ego network and one
+//     pivot for all roots of a vertex (run_vertex); small vertices of large
+//     graphs are decided 32 to a warp before that (tiny.cu).
 //   * Root-down exposure with self-contained tasks.  When warps are idle, a
 //     busy warp turns every open candidate of the shallowest open level with
 //     |P| >= tau -- outer tiers of a nested solve first -- into a task record
