@@ -3122,12 +3122,12 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && nwork;
   if (plan->vertex_pass) {
     P.edge_out = (uint32_t *)scr->get(8, nwork * 4, &s);
-    if (!P.edge_out) return s;
+    plan->vertex_pass = P.edge_out != nullptr;  // no room for the list: root by root
     P.edge_n = &ctl->edge_n;
-    P.vertex_pass = 1;
-    if (g.n > kVertexSingles * nwarps) {
-      P.vert_list = (uint32_t *)scr->get(9, (uint64_t)g.n * 4, &s);
-      if (!P.vert_list) return s;
+    P.vertex_pass = plan->vertex_pass;
+    if (plan->vertex_pass && g.n > kVertexSingles * nwarps) P.vert_list = (uint32_t *)scr->get(9, (uint64_t)g.n * 4, &s);
+    s = MCE_OK;
+    if (P.vert_list) {
       P.vert_n = &ctl->vert_n;
       P.single_items = kVertexSingles * nwarps;
     }
