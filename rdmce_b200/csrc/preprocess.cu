@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "barrier.h"
 #include "common.cuh"
 #include "engine.h"
 
@@ -156,7 +157,7 @@ __global__ void k_iota(uint32_t *a, uint64_t n) {
 // Measured (B200): R-MAT 20 (192 levels, 622 rounds) 5.3 -> 4.1 ms, the core below
 // included.
 struct PeelCtl {
-  uint32_t arrived;     // barrier arrivals so far
+  uint32_t arrived;     // kBarrierStart + barrier arrivals so far
   uint32_t degeneracy;
   uint32_t rounds;
   uint32_t levels;
@@ -184,8 +185,8 @@ __device__ __forceinline__ bool grid_barrier(PeelCtl *ctl, uint32_t *target, uin
     uint64_t n = 0;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&ctl->arrived) : "memory");
-    } while (seen < *target && ++n < spin_limit);
-    ok = seen >= *target;
+    } while (!barrier_reached(seen, *target) && ++n < spin_limit);
+    ok = barrier_reached(seen, *target);
     if (!ok) atomicExch(&ctl->error, 2u);
   }
   __syncthreads();
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(kPeelThreads) k_peel_rounds(uint32_t n, const 
   const bool leader = tid == 0;
   __shared__ uint32_t s_at[2][kPeelThreads / 32], s_min[kPeelThreads / 32];
   __shared__ unsigned long long s_sum[kPeelThreads / 32];
-  uint32_t target = 0;
+  uint32_t target = kBarrierStart;
   uint32_t k = 0, degen = 0, lev = 0, r = 0, removed = 0, nrem = n;
   uint32_t *rem_cur = remA, *rem_nxt = remB;
   while (removed < n) {
@@ -676,6 +677,7 @@ mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint
   // build (and unpinning, which synchronises the device) would stall other
   // streams' work, e.g. concurrently served requests
   PeelCtl h{};
+  h.arrived = kBarrierStart;
   PeelCtl *hc = &h;
   if (core_only) h.nrem = n;
   MCE_CUDA_TRY(cudaMemcpyAsync(ctl.p, hc, sizeof(PeelCtl), cudaMemcpyHostToDevice, st));
