@@ -178,7 +178,7 @@ struct EnumParams {
   unsigned long long *stat_bbytes;       // algorithmic ego-network build bytes (stats mode)
   unsigned long long *stat_cycles;       // per phase: build, 64-bit tier, general tier, spawn, idle, queue, 32-bit tier
   unsigned long long *stat_max_item;     // [2]: longest root, longest task, in cycles
-  unsigned int *active;                  // warps holding work
+  unsigned int *active;                  // warps that may claim items, and unfinished tasks
   // task pool: blocks of block_bytes, a free ring and a ready ring (one cell per block)
   char *pool;
   uint32_t block_bytes;

@@ -362,13 +362,16 @@ __device__ __forceinline__ void pool_free(const Ctx &c, uint32_t blk) {
   __syncwarp();
 }
 
+// A task counts as busy from before it is published until its taker has
+// finished it (see idle_wait).
 __device__ __forceinline__ void pool_publish(const Ctx &c, uint32_t blk) {
   const EnumParams &P = *c.P;
   __threadfence();
   __syncwarp();
   if (c.lane == 0) {
+    atomicAdd(P.active, 1u);
     __threadfence();
-    ring_push(P.ready_slot, P.ready_seq, P.ready_tail, P.ready_count, P.pool_mask, blk, P);
+    if (!ring_push(P.ready_slot, P.ready_seq, P.ready_tail, P.ready_count, P.pool_mask, blk, P)) atomicSub(P.active, 1u);
     atomicAdd(P.stat_tasks, 1ULL);
   }
   __syncwarp();
@@ -378,16 +381,11 @@ __device__ __forceinline__ char *pool_block(const EnumParams &P, uint32_t blk) {
   return P.pool + (uint64_t)blk * P.block_bytes;
 }
 
-// busy warps expose work when some warps are idle and the queue is short
+// busy warps expose work while fewer tasks are queued than warps are idle
 __device__ __forceinline__ bool hungry(const Ctx &c) {
   const EnumParams &P = *c.P;
   uint32_t h = 0;
-  if (c.lane == 0) {
-    const uint32_t active = *(volatile unsigned int *)P.active;
-    const int queued = *(volatile int *)P.ready_count;
-    const int idle = (int)P.nwarps - (int)active;
-    h = idle > 0 && queued < idle;
-  }
+  if (c.lane == 0) h = *(volatile unsigned int *)P.active < P.nwarps;
   return __shfl_sync(kFull, h, 0) != 0;
 }
 
@@ -2777,27 +2775,28 @@ __device__ __noinline__ void run_root(Ctx c, uint64_t k) {
 }
 
 // Wait for a task while other warps are busy.  Returns a pool block taken
-// from the ready queue (the warp then counts as busy), or -1 when no work is
+// from the ready queue (it counts as busy until its taker ends it), or -1 when no work is
 // left anywhere (or the wait's bound ran out: the error word says so).
 //
 // At most one warp per block polls the global queue at a time (the block's
-// poll token); the others sleep.  A task is published before its producer
-// stops counting as busy, and a taker counts itself busy before it takes, so a
-// task is in the queue's count or its warp in the busy count at any time.  "No
-// work left" is nobody busy, queue empty, nobody busy: with only one look at
-// the busy count, before the queue's, a task taken between the two was missed,
-// and where one task hopped from warp to warp (the narrow top of a deep tree)
-// half of the blocks left before the work it still held came out: full R-MAT
-// 14 then ran its second half on 1600 of 3552 warps (25 ms instead of 16).
-// Exit waits for two such observations a back-off apart; the block's other
-// warps then leave with the poller (token value 2), instead of each waiting
-// for its own two.  Not inlined, so its loop holds only a few values: idle
-// polling costs no reloads of the caller's state.
+// poll token); the others sleep.  The busy count holds every warp that may
+// still claim an item and every task from before it is published until its
+// taker has finished it.  Whoever adds to it is counted already (a task's
+// producer; a warp before its first claim), so zero in this one word means that
+// no task is queued or held: one look is enough, in any order of the ring's
+// own counts.  (Warps that start late count themselves in, and wait for zero
+// like any other before they leave.)  A count of busy warps alone needs the
+// queue's count beside it, and no order of looks at the two sees a task that
+// hops from warp to warp: blocks then left before the work it still held came
+// out (full R-MAT 14 ran its second half on 1600 of 3552 warps, 25 ms instead
+// of 16), and could leave a task behind.  The poller that sees zero leaves
+// token value 2: the block's other warps look at the busy count themselves and
+// leave, instead of each waiting for its turn.  Not inlined, so its loop holds
+// only a few values: idle polling costs no reloads of the caller's state.
 __device__ __noinline__ int idle_wait(Ctx c, unsigned int *s_poll) {
   const EnumParams &P = *c.P;
   WarpSmem *sm = c.sm;
   uint64_t idle_spins = 0;
-  uint32_t quiet = 0;  // consecutive "nobody busy, queue empty" observations
   for (;;) {
     int result = -2;  // -2: keep waiting
     if (c.lane == 0) {
@@ -2805,26 +2804,16 @@ __device__ __noinline__ int idle_wait(Ctx c, unsigned int *s_poll) {
       bool polled = false, seen = false;
       const unsigned int token = atomicCAS(s_poll, 0u, 1u);
       if (token == 2u) {
-        result = -1;
+        if (*(volatile unsigned int *)P.active == 0) result = -1;
+        else atomicCAS(s_poll, 2u, 0u);  // a warp that started late holds work
       } else if (token == 0u) {
         polled = true;
-        const uint32_t act = *(volatile unsigned int *)P.active;
-        __threadfence();
-        if (*(volatile int *)P.ready_count > 0) {
+        if (*(volatile unsigned int *)P.active == 0) {
+          result = -1;
+        } else if (*(volatile int *)P.ready_count > 0) {
           seen = true;
           uint32_t b = 0;
-          atomicAdd(P.active, 1u);
-          __threadfence();
           if (ring_pop(P.ready_slot, P.ready_seq, P.ready_head, P.ready_count, P.pool_mask, &b, P)) result = (int)b;
-          else atomicSub(P.active, 1u);
-          quiet = 0;
-        } else {
-          __threadfence();
-          if (act == 0 && *(volatile unsigned int *)P.active == 0) {
-            if (++quiet >= 2) result = -1;
-          } else {
-            quiet = 0;
-          }
         }
         atomicExch(s_poll, result == -1 ? 2u : 0u);
       }
@@ -2897,7 +2886,10 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
       if (got) {
         const unsigned long long tb = now();
         solve_block(c, blk);
-        if (c.lane == 0) atomicMax(P.stat_max_item + 1, now() - tb);
+        if (c.lane == 0) {
+          atomicMax(P.stat_max_item + 1, now() - tb);
+          atomicSub(P.active, 1u);
+        }
         continue;
       }
     }
@@ -3174,8 +3166,10 @@ mce_status MCE_ENUM_FN(enum_finish)(const EnumPlan &plan, cudaStream_t st, EnumS
   uint64_t cycles[kCycPhases];
   for (int i = 0; i < kCycPhases; i++) cycles[i] = h.stat_cycles[i];
   uint64_t max_item[2] = {h.stat_max_item[0], h.stat_max_item[1]};
-  uint32_t err = h.error;
-  if (h.heavy_n && !h.error) {
+  // 5: a task was left behind (cannot happen, see idle_wait): the totals are short
+  const auto error_of = [](const EnumCtl &x) { return x.error ? x.error : x.active || x.ready_count ? 5u : 0u; };
+  uint32_t err = error_of(h);
+  if (h.heavy_n && !err) {
     // Deferred roots: one slab per warp, each sized for the largest deferred
     // ego network; every warp of the pass shares their work (unless per-root
     // values are being attributed, which keeps each root on one warp).  Only
@@ -3238,7 +3232,7 @@ mce_status MCE_ENUM_FN(enum_finish)(const EnumPlan &plan, cudaStream_t st, EnumS
     bbytes += h2.stat_bbytes;
     for (int i = 0; i < kCycPhases; i++) cycles[i] += h2.stat_cycles[i];
     for (int i = 0; i < 2; i++) max_item[i] = std::max<uint64_t>(max_item[i], h2.stat_max_item[i]);
-    err = h2.error;
+    err = error_of(h2);
   }
   if (stats) {
     stats->roots = roots;
@@ -3254,6 +3248,7 @@ mce_status MCE_ENUM_FN(enum_finish)(const EnumPlan &plan, cudaStream_t st, EnumS
   }
   if (err == 2) return MCE_ERR_OUT_OF_MEMORY;
   if (err == 4) return MCE_ERR_CAPACITY;
+  if (err == 5) return MCE_ERR_INTERNAL;
   if (err) return MCE_ERR_TIMEOUT;
   return MCE_OK;
 }
