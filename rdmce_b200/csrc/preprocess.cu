@@ -170,6 +170,10 @@ struct PeelCtl {
 // memory and is worth few enough neighbour visits.
 constexpr uint32_t kCoreVertices = 16384, kCoreEntries = 3u << 20;
 constexpr uint32_t kPeelThreads = 512;
+// A barrier waits for the other blocks' share of a round, which is work that
+// ends, so a caller's limit on idle polls does not cut it short: at least this
+// many polls, most of a minute.
+constexpr uint64_t kPeelSpinMin = 1ULL << 26;
 constexpr uint32_t kPeelAsk = 256;  // frontiers from this size on skip removed neighbours (atomics bound them)
 
 // One barrier of the whole grid (all blocks are resident); false when the wait
@@ -663,6 +667,7 @@ mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint
   k_iota<<<grid_for(n, 256), 256, 0, st>>>(remA.p, n); note_launch();
   // one counter a round (every round but the last of a level claims a vertex)
   // and two a level
+  spin_limit = std::max(spin_limit, kPeelSpinMin);
   const uint64_t max_levels = (uint64_t)max_degree + 2, max_rounds = (uint64_t)n + max_levels + 4;
   const bool core_only = n <= kCoreVertices && entries <= kCoreEntries;
   DevBuf<uint32_t> counters;
