@@ -59,6 +59,15 @@ struct Flat {
 // A vertex is taken here with 1 to kTinyP later neighbours and up to
 // kTinyDegree neighbours (its earlier ones are visited too).
 constexpr uint32_t kTinyP = 8, kTinyDegree = 256, kTinyWarps = 8;
+// An earlier neighbour's list is walked from its end for this many elements,
+// then searched for the later neighbours not yet passed.  In a degeneracy order
+// few of its neighbours come after v and the walk ends first; in the other
+// orders a hub comes early and has nearly its whole list there.
+// Measured (B200), enumeration: a hub of 200,000 neighbours with 1 and 7 later
+// neighbours each (stored order) 60 and 237 ms walked to the end, 1.05 and 1.51
+// here, 1.15 and 1.93 with 256 elements; searching from the first element on,
+// G(10^6, mean degree 6) takes 0.33 ms instead of 0.30.
+constexpr uint32_t kTinyWalk = 16;
 
 // A set of later neighbours is a lane number (the first five) and a group (the
 // others); the sets of one group are one 32-bit word.
@@ -111,6 +120,11 @@ __device__ uint64_t tiny_vertex(const DevGraph &g, TinyWarp *ts, uint32_t v, uin
         uint32_t m = 0, e = ue, k = n, c = __ldg(g.adj + base + n - 1);
         const uint32_t least = __ldg(g.adj + base);
         while (e > ub && k) {
+          if (ue - e == kTinyWalk) {  // many neighbours after v: search them for the others
+            for (uint32_t i = 0; i < k; i++)
+              if (contains_u32(g.adj + ub, e - ub, __ldg(g.adj + base + i))) m |= 1u << i;
+            break;
+          }
           const uint32_t y = __ldg(g.adj + e - 1);
           if (y < least) break;
           while (k && c > y) {

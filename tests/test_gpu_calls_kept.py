@@ -23,3 +23,22 @@ def test_graph_build_with_the_smallest_wait_limit(gpu, oracle_mod):
         assert g.info()["degeneracy"] == og.degeneracy
     off, adj, olab = og.export()
     assert np.array_equal(ro.astype(np.uint64), off) and np.array_equal(ci, adj) and np.array_equal(lab, olab)
+
+
+def test_light_vertices_of_an_early_hub(gpu, oracle_mod):
+    """In the stored order a hub comes first and nearly all its neighbours come
+    after each of its light neighbours; these must not walk its whole list (the
+    degeneracy order, where the hub comes last, takes about a fifth of the time)."""
+    D, later = 200000, 7
+    i = np.arange(1, D + 1, dtype=np.uint32)
+    u = np.concatenate([np.zeros(D, np.uint32)] + [i[:-s] for s in range(1, later + 1)])
+    v = np.concatenate([i] + [i[s:] for s in range(1, later + 1)])
+    o = oracle_mod.Graph.from_pairs(u, v).sort_degeneracy().mce(threads=THREADS)
+    ms = {}
+    for order in (gpu.ORDER_UNCHANGED, gpu.ORDER_DEGREE_DESC, gpu.ORDER_DEGENERACY):
+        with gpu.Graph.from_coo(u, v, opts(gpu, order=order)) as g:
+            runs = [g.solve(opts(gpu, blocks_per_sm=4)) for _ in range(5)]
+        for r in runs:
+            assert (r.count, r.checksum, r.hist, r.max_size) == (o.count, o.checksum, o.hist, o.max_size)
+        ms[order] = min(r.phase_ms[3] for r in runs)
+    assert max(ms.values()) < 50 * ms[gpu.ORDER_DEGENERACY], ms
