@@ -144,7 +144,7 @@ struct EnumParams {
   const uint64_t *root_list;             // list mode: root ids (else the range [rb, re))
   uint64_t n_list;                       // entries in root_list
   int vertex_pass;                       // work items are the vertices of the range, not its roots
-  uint32_t *vert_list;                   // vertex pass: after the last single_items vertices, those to take (null: all)
+  uint32_t *vert_list;                   // vertex pass: of the vertices before the graph's last single_items, those to take (null: all)
   uint64_t single_items;
   unsigned int *vert_n;                  // how many
   uint32_t *edge_out;                    // vertex pass: roots left to the edge pass
@@ -189,6 +189,25 @@ struct EnumParams {
   int *free_count, *ready_count;         // filled cells not yet claimed
 };
 
+#ifdef __CUDACC__
+// The vertices of a root range: roots are in vertex order, so they are one
+// interval, and a range that is narrow against the graph visits no others.
+// Measured (B200), the enumeration of 10 roots: 0.80 -> 0.05 ms against visiting
+// all vertices in 50,000,000 separate edges, 0.10 -> 0.05 ms in G(5e6, mean
+// degree 4).
+__device__ __forceinline__ uint32_t range_last(const EnumParams &P) { return P.g.root_v0[P.re - 1]; }
+__device__ __forceinline__ uint32_t range_vertices(const EnumParams &P) {
+  return range_last(P) - P.g.root_v0[P.rb] + 1;
+}
+// How many of them are items in order: those among the graph's last
+// single_items, all without a list.
+__device__ __forceinline__ uint32_t range_singles(const EnumParams &P) {
+  const uint32_t items = range_vertices(P);
+  if (!P.vert_list) return items;
+  const uint64_t above = (uint64_t)range_last(P) + 1 + P.single_items;
+  return above > P.g.n ? (uint32_t)min((uint64_t)items, above - P.g.n) : 0;
+}
+#endif
 
 // A planned enumeration: scratch allocated, launch shape fixed.  Launch may be
 // captured into a CUDA graph; finish reads the control words and runs the

@@ -2624,7 +2624,8 @@ __device__ __noinline__ uint32_t run_vertex(Ctx c, uint64_t k) {
   const EnumParams &P = *c.P;
   const DevGraph &g = P.g;
   // late-peeled vertices first: they are the heavy ones
-  const uint32_t v = P.vert_list && k >= P.single_items ? P.vert_list[k - P.single_items] : g.n - 1 - (uint32_t)k;
+  const uint32_t singles = range_singles(P);
+  const uint32_t v = k < singles ? range_last(P) - (uint32_t)k : P.vert_list[k - singles];
   const uint32_t r0 = g.root_off[v], r1 = g.root_off[v + 1];
   const uint32_t lo = (uint32_t)max((uint64_t)r0, P.rb), hi = (uint32_t)min((uint64_t)r1, P.re);
   if (lo >= hi) return 0;
@@ -2864,7 +2865,7 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
   c.sharing = P.sharing != 0;
   if (P.edge_list && !P.heavy_list && *P.edge_n == 0) return;  // the vertex pass left nothing (all blocks agree)
   const uint64_t total = P.heavy_list    ? P.n_heavy
-                         : P.vertex_pass ? (P.vert_list ? P.single_items + *P.vert_n : P.g.n)
+                         : P.vertex_pass ? range_singles(P) + (uint64_t)(P.vert_list ? *P.vert_n : 0)
                          : P.edge_list   ? *P.edge_n
                          : P.root_list   ? P.n_list
                                          : P.re - P.rb;

@@ -9,7 +9,8 @@
 // later neighbours and the earlier neighbours of all of them are flattened
 // over the lanes, and every lane then decides its own vertex on words of
 // subsets.  The other vertices are listed for the enumeration kernel (enum.cu),
-// which takes the last P.single_items vertices of the order itself.
+// which takes the last P.single_items vertices of the order itself.  A root
+// range is its vertices' interval (range_vertices).
 // Measured (B200): Chung-Lu 10^6 (mean degree 16) enumeration 7.3 -> 6.4 ms.
 #include <algorithm>
 
@@ -235,11 +236,12 @@ __global__ void __launch_bounds__(32 * kTinyWarps) k_tiny(const __grid_constant_
   uint64_t chk = 0;
   unsigned long long roots = 0;
   const uint32_t nwarps = gridDim.x * kTinyWarps;
-  for (uint64_t k = P.single_items + (uint64_t)(blockIdx.x * kTinyWarps + wid) * 32; k < g.n; k += (uint64_t)nwarps * 32) {
+  const uint32_t last = range_last(P), items = range_vertices(P);
+  for (uint64_t k = range_singles(P) + (uint64_t)(blockIdx.x * kTinyWarps + wid) * 32; k < items; k += (uint64_t)nwarps * 32) {
     uint32_t v = 0, b = 0, d = 0, p = 0;
     bool left = false, tiny = false;
-    if (k + lane < g.n) {
-      v = g.n - 1 - (uint32_t)(k + lane);
+    if (k + lane < items) {
+      v = last - (uint32_t)(k + lane);
       const uint32_t r0 = g.root_off[v], r1 = g.root_off[v + 1];
       b = g.off[v];
       d = g.off[v + 1] - b;

@@ -42,3 +42,18 @@ def test_light_vertices_of_an_early_hub(gpu, oracle_mod):
             assert (r.count, r.checksum, r.hist, r.max_size) == (o.count, o.checksum, o.hist, o.max_size)
         ms[order] = min(r.phase_ms[3] for r in runs)
     assert max(ms.values()) < 50 * ms[gpu.ORDER_DEGENERACY], ms
+
+
+def test_narrow_root_range_of_a_large_graph(gpu):
+    """A few roots of 10^8 vertices cost what they cost in a small graph: a
+    range visits its own vertices, not all of them."""
+    ms = {}
+    for pairs in (100_000, 50_000_000):
+        u = np.arange(0, 2 * pairs, 2, dtype=np.uint32)
+        with gpu.Graph.from_coo(u, u + 1, opts(gpu)) as g:
+            assert g.info()["num_edges"] == pairs
+            for begin in (0, pairs // 2, pairs - 10):
+                runs = [g.solve(opts(gpu, blocks_per_sm=4, root_begin=begin, root_end=begin + 10)) for _ in range(15)]
+                assert all((r.count, r.roots, r.hist) == (10, 10, {2: 10}) for r in runs)
+                ms.setdefault(pairs, []).append(min(r.phase_ms[3] for r in runs))
+    assert max(ms[50_000_000]) < 1.5 * max(ms[100_000]), ms
