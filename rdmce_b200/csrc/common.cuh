@@ -6,6 +6,7 @@
 #include <cstdio>
 
 #include "internal.h"
+#include "scratch.h"
 
 #define MCE_CUDA_TRY(expr)                                   \
   do {                                                       \
@@ -114,27 +115,6 @@ mce_status radix_sort_u64(uint64_t *&keys, uint64_t *&tmp, uint64_t n, int lo, i
 mce_status csr_offsets_static(int device, const uint32_t *deg, uint32_t *off, uint64_t n, cudaStream_t st);
 // reduce max of n uint32
 mce_status reduce_max_u32(const uint32_t *in, uint64_t n, uint32_t *d_out, cudaStream_t st);
-
-// Device scratch owned by one solver context: buffers keyed by purpose, grown
-// on demand and kept for reuse (the role of the reference's BufferManager,
-// include/context_gpu.cuh:4-32, without its worst-case sizing).
-struct Scratch {
-  static constexpr int kSlots = 10;
-  int device = 0;
-  // set: buffers are allocated and freed stream-ordered on this stream (no
-  // device-wide synchronisation when one grows), for an owner whose work
-  // stays on that stream (a server dispatcher)
-  cudaStream_t ordered = nullptr;
-  void *ptr[kSlots] = {};
-  size_t bytes[kSlots] = {};
-  void *get(int purpose, size_t n, mce_status *st);
-  void release();
-  ~Scratch() { release(); }
-};
-// the default per-device context used by single-graph calls, and its lock
-Scratch *default_scratch(int device);
-void lock_default(int device);
-void unlock_default(int device);
 
 // every kernel launch of the engine is counted (mce_launch_count)
 void note_launch();

@@ -3079,13 +3079,23 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   plan->fits_all = slab_bytes >= bound;
   char *slab = (char *)scr->get(2, slab_bytes * nwarps, &s);
   if (!slab) return s;
-  // roots whose ego network overflows the slab are deferred to a second pass;
-  // the list holds their work indices (a solve of more than 2^32 roots is
-  // refused by the callers)
+  // A range goes vertex by vertex first; per-root values and the counters of
+  // the edge-rooted method (stats) need every root on its own.
+  plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && nwork;
+  // One buffer of lists: the vertex pass's roots and vertices left, and the
+  // roots whose ego network overflows the slab, deferred to a second pass.
+  // Those are kept by work index (a solve of more than 2^32 roots is refused by
+  // the callers).  One buffer, since each that grows with the graph costs a
+  // first solve an allocation, which waits for the device.
   const uint64_t heavy_cap = std::min<uint64_t>(nwork, 1ULL << 26);
   uint32_t *heavy = nullptr;
   if (nwork) {
-    heavy = (uint32_t *)scr->get(3, heavy_cap * 4, &s);
+    const uint64_t pass = plan->vertex_pass ? nwork + g.n : 0;
+    heavy = (uint32_t *)scr->get(3, (heavy_cap + pass) * 4, &s);
+    if (!heavy && pass) {  // no room for the vertex pass's lists: root by root
+      plan->vertex_pass = false;
+      heavy = (uint32_t *)scr->get(3, heavy_cap * 4, &s);
+    }
     if (!heavy) return s;
   }
   // task pool: one record per block; both rings have one cell per block
@@ -3110,17 +3120,12 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   P.re = re;
   P.root_list = list_mode ? cfg.root_list : nullptr;
   P.n_list = list_mode ? cfg.n_root_list : 0;
-  // A range goes vertex by vertex first; per-root values and the counters of
-  // the edge-rooted method (stats) need every root on its own.
-  plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && nwork;
   if (plan->vertex_pass) {
-    P.edge_out = (uint32_t *)scr->get(8, nwork * 4, &s);
-    plan->vertex_pass = P.edge_out != nullptr;  // no room for the list: root by root
+    P.vertex_pass = 1;
+    P.edge_out = heavy + heavy_cap;
     P.edge_n = &ctl->edge_n;
-    P.vertex_pass = plan->vertex_pass;
-    if (plan->vertex_pass && g.n > kVertexSingles * nwarps) P.vert_list = (uint32_t *)scr->get(9, (uint64_t)g.n * 4, &s);
-    s = MCE_OK;
-    if (P.vert_list) {
+    if (g.n > kVertexSingles * nwarps) {
+      P.vert_list = P.edge_out + nwork;
       P.vert_n = &ctl->vert_n;
       P.single_items = kVertexSingles * nwarps;
     }

@@ -364,8 +364,9 @@ void *Scratch::get(int purpose, size_t n, mce_status *st) {
   }
   ptr[purpose] = nullptr;
   bytes[purpose] = 0;
-  const cudaError_t e = ordered ? cudaMallocAsync(&ptr[purpose], std::max<size_t>(n, 256), ordered)
-                                : cudaMalloc(&ptr[purpose], std::max<size_t>(n, 256));
+  const cudaError_t e = most[purpose] && n > most[purpose] ? cudaErrorMemoryAllocation
+                        : ordered ? cudaMallocAsync(&ptr[purpose], std::max<size_t>(n, 256), ordered)
+                                  : cudaMalloc(&ptr[purpose], std::max<size_t>(n, 256));
   if (e != cudaSuccess) {
     cudaGetLastError();
     ptr[purpose] = nullptr;

@@ -2,11 +2,13 @@
 from __future__ import annotations
 
 import os
+import shutil
+import subprocess
 
 import numpy as np
 import pytest
 
-from conftest import opts
+from conftest import ROOT, opts
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +59,19 @@ def test_narrow_root_range_of_a_large_graph(gpu):
                 assert all((r.count, r.roots, r.hist) == (10, 10, {2: 10}) for r in runs)
                 ms.setdefault(pairs, []).append(min(r.phase_ms[3] for r in runs))
     assert max(ms[50_000_000]) < 1.5 * max(ms[100_000]), ms
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="no host C++ compiler")
+def test_no_room_for_the_vertex_pass(gpu, oracle_mod, tmp_path):
+    """Where the vertex pass's lists cannot be allocated, a range goes root by root."""
+    u, v = gpu.gen_gnp(60000, 9.0, 17)  # more vertices than warps take singly
+    o = oracle_mod.Graph.from_pairs(u, v).sort_degeneracy().mce(threads=THREADS)
+    path, exe = str(tmp_path / "pairs"), str(tmp_path / "scratch_check")
+    np.concatenate([u, v]).tofile(path)
+    lib = os.path.join(ROOT, "rdmce_b200")
+    subprocess.run(["g++", "-O1", "-std=c++17", f"-I{os.path.join(lib, 'csrc')}", f"-I{os.path.join(ROOT, 'include')}",
+                    "-I/usr/local/cuda/include", os.path.join(ROOT, "tests", "cpp", "scratch_check.cc"), f"-L{lib}",
+                    "-lrdmce", f"-Wl,-rpath,{lib}", "-lpthread", "-o", exe], check=True, timeout=300)
+    r = subprocess.run([exe, path, str(len(u))], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert f"SCRATCH OK count {o.count} checksum {o.checksum}" in r.stdout
