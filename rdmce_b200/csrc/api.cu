@@ -341,7 +341,8 @@ mce_status mce_graph_info_get(const mce_graph *g, mce_graph_info *info) {
   info->num_edges = g->g.m;
   info->max_degree = g->g.max_degree;
   info->degeneracy = g->g.degeneracy;
-  info->device_bytes = (uint64_t)(g->g.n + 1) * 4 + 2 * g->g.m * 4 + (uint64_t)g->g.n * (4 + 16) + g->g.m * 8;
+  // offsets and first roots; adjacency; labels and their hashes; roots
+  info->device_bytes = ((uint64_t)g->g.n + 1) * (4 + 4) + 2 * g->g.m * 4 + (uint64_t)g->g.n * (4 + 16) + g->g.m * 8;
   return MCE_OK;
 }
 

@@ -75,3 +75,12 @@ def test_no_room_for_the_vertex_pass(gpu, oracle_mod, tmp_path):
     r = subprocess.run([exe, path, str(len(u))], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert f"SCRATCH OK count {o.count} checksum {o.checksum}" in r.stdout
+
+
+def test_device_bytes_counts_every_array(gpu):
+    """Offsets, first roots, adjacency, labels with two hashes, root pairs."""
+    u, v = gpu.gen_gnp(5000, 7.0, 3)
+    with gpu.Graph.from_coo(u, v, opts(gpu)) as g:
+        i = g.info()
+        n, m = i["num_vertices"], i["num_edges"]
+        assert i["device_bytes"] == 4 * (n + 1) + 4 * (n + 1) + 8 * m + (4 + 8 + 8) * n + 8 * m
