@@ -106,8 +106,8 @@ __global__ void k_run_degrees(const uint32_t *ub, const uint32_t *ue, const uint
     deg[v] = (ue[v] - ub[v]) + (le[v] - lb[v]);
 }
 
-// Row r of vertex v starts at off[r]; its smaller neighbours come first.  The
-// element at position i of a sorted edge list goes to i + (the list's base of
+// Row r of vertex v (rank[v], or v without ranks) starts at off[r]; its smaller
+// neighbours come first.  The element at position i of a sorted edge list goes to i + (the list's base of
 // v), modulo 2^32.
 __global__ void k_run_bases(const uint32_t *off, const uint32_t *rank, const uint32_t *ub, const uint32_t *lb,
                             const uint32_t *le, uint32_t n, uint32_t *ubase, uint32_t *lbase) {
@@ -115,6 +115,17 @@ __global__ void k_run_bases(const uint32_t *off, const uint32_t *rank, const uin
     const uint32_t o = off[rank ? rank[v] : v];
     lbase[v] = o - lb[v];
     ubase[v] = o + (le[v] - lb[v]) - ub[v];
+  }
+}
+
+// The bases for rows that start at off_new[rank[v]] instead of off_old[v]: with
+// them the runs' bounds, four words a vertex, need not be kept while peeling.
+__global__ void k_move_bases(const uint32_t *off_old, const uint32_t *off_new, const uint32_t *rank, uint32_t n,
+                             uint32_t *ubase, uint32_t *lbase) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const uint32_t by = off_new[rank[v]] - off_old[v];
+    lbase[v] += by;
+    ubase[v] += by;
   }
 }
 
@@ -648,9 +659,9 @@ mce_status read_scalar(const T *d, T *h, cudaStream_t st) {
   return MCE_OK;
 }
 
-// k-core peeling over an unsorted symmetric CSR; fills order[] (position -> vertex)
+// k-core peeling over an unsorted symmetric CSR; allocates and fills order[] (position -> vertex)
 mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint32_t *deg0, uint32_t max_degree,
-                uint64_t entries, uint32_t *order, uint32_t *degeneracy, uint64_t spin_limit, cudaStream_t st) {
+                uint64_t entries, DevBuf<uint32_t> &order, uint32_t *degeneracy, uint64_t spin_limit, cudaStream_t st) {
   DevBuf<int> deg;
   DevBuf<uint32_t> state, remA, remB;
   DevBuf<uint2> frA, frB;
@@ -735,7 +746,8 @@ mce_status peel(uint32_t n, const uint32_t *off, const uint32_t *adj, const uint
   k_round_keys<<<grid_for(n, 256), 256, 0, st>>>(state.p, n, nb, keys.p); note_launch();
   // the keys are in vertex order already: a stable sort by round finishes them
   MCE_TRY(radix_sort_u64(keys.p, tmp.p, n, nb, nb + rb_bits, st));
-  k_order_from_round_keys<<<grid_for(n, 256), 256, 0, st>>>(keys.p, n, (1ULL << nb) - 1, order); note_launch();
+  MCE_TRY(order.alloc(n, st));
+  k_order_from_round_keys<<<grid_for(n, 256), 256, 0, st>>>(keys.p, n, (1ULL << nb) - 1, order.p); note_launch();
   MCE_CUDA_TRY(cudaGetLastError());
   return MCE_OK;
 }
@@ -941,28 +953,30 @@ mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32
   MCE_TRY(read_scalar(maxd.p, &g->max_degree, st));
 
   // 3) vertex order
-  DevBuf<uint32_t> order, rank;
-  MCE_TRY(order.alloc(n, st));
-  MCE_TRY(rank.alloc(n, st));
+  DevBuf<uint32_t> order, rank, off0;  // off0: row starts under the old ids, degeneracy order only
   g->degeneracy = g->max_degree;  // Graph::LoadFromFile leaves degeneracy_ = max degree (graph.cc:149)
   if (order_kind == MCE_ORDER_DEGENERACY && n > 0) {
-    DevBuf<uint32_t> off0, adj0;
+    DevBuf<uint32_t> adj0;
     MCE_TRY(off0.alloc(n + 1, st));
     MCE_TRY(adj0.alloc(m2, st));
     MCE_TRY(scan_exclusive_u32(deg.p, off0.p, n, off0.p + n, st));
     k_run_bases<<<grid_for(n, 256), 256, 0, st>>>(off0.p, nullptr, ub, lb, le, n, ubase, lbase); note_launch();
+    runs.release();
     k_fill_adj<<<grid_for(m, 256), 256, 0, st>>>(eu, ev, by_v.p, m, nb, ubase, lbase, adj0.p); note_launch();
-    MCE_TRY(peel(n, off0.p, adj0.p, deg.p, g->max_degree, m2, order.p, &g->degeneracy, spin_limit, st));
+    MCE_TRY(peel(n, off0.p, adj0.p, deg.p, g->max_degree, m2, order, &g->degeneracy, spin_limit, st));
   } else if ((order_kind == MCE_ORDER_DEGREE_ASC || order_kind == MCE_ORDER_DEGREE_DESC) && n > 0) {
     DevBuf<uint64_t> dk, dt;
     MCE_TRY(dk.alloc(n, st));
     MCE_TRY(dt.alloc(n, st));
     k_degree_keys<<<grid_for(n, 256), 256, 0, st>>>(deg.p, n, order_kind == MCE_ORDER_DEGREE_DESC, dk.p); note_launch();
     MCE_TRY(radix_sort_u64(dk.p, dt.p, n, 0, 64, st));
+    MCE_TRY(order.alloc(n, st));
     k_order_from_keys<<<grid_for(n, 256), 256, 0, st>>>(dk.p, n, order.p); note_launch();
   } else {
+    MCE_TRY(order.alloc(n, st));
     k_iota<<<grid_for(n, 256), 256, 0, st>>>(order.p, n); note_launch();
   }
+  MCE_TRY(rank.alloc(n, st));
   k_rank_from_order<<<grid_for(n, 256), 256, 0, st>>>(order.p, n, rank.p); note_launch();
   order.release();
 
@@ -975,7 +989,11 @@ mce_status finish_graph(uint32_t n, uint64_t m, const uint32_t *eu, const uint32
   k_permute_degrees<<<grid_for(n, 256), 256, 0, st>>>(deg.p, rank.p, n, deg_new.p); note_launch();
   MCE_CUDA_TRY(cudaMallocAsync(&g->off, (n + 1) * sizeof(uint32_t), st));
   MCE_TRY(scan_exclusive_u32(deg_new.p, g->off, n, g->off + n, st));
-  k_run_bases<<<grid_for(n, 256), 256, 0, st>>>(g->off, rank.p, ub, lb, le, n, ubase, lbase); note_launch();
+  if (off0.p) {
+    k_move_bases<<<grid_for(n, 256), 256, 0, st>>>(off0.p, g->off, rank.p, n, ubase, lbase); note_launch();
+  } else {
+    k_run_bases<<<grid_for(n, 256), 256, 0, st>>>(g->off, rank.p, ub, lb, le, n, ubase, lbase); note_launch();
+  }
   k_relabel_keys<<<grid_for(m, 256), 256, 0, st>>>(eu, ev, by_v.p, m, rank.p, ubase, lbase, nb, keys.p); note_launch();
   by_v.release();
   MCE_TRY(radix_sort_u64(keys.p, tmp.p, m2, nb, 2 * nb, st));

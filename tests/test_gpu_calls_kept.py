@@ -84,3 +84,31 @@ def test_device_bytes_counts_every_array(gpu):
         i = g.info()
         n, m = i["num_vertices"], i["num_edges"]
         assert i["device_bytes"] == 4 * (n + 1) + 4 * (n + 1) + 8 * m + (4 + 8 + 8) * n + 8 * m
+
+
+def used_at_most(gpu, u, v):
+    """The most device memory a build held, stream-ordered allocations of the default pool."""
+    import ctypes as C
+
+    cu, pool, value = C.CDLL("libcuda.so.1"), C.c_void_p(), C.c_uint64(0)
+    used_now, used_high = 7, 8  # CU_MEMPOOL_ATTR_USED_MEM_CURRENT, _HIGH
+    gpu.Graph.from_coo(u[:10], v[:10], opts(gpu)).close()
+    assert cu.cuDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+    assert cu.cuMemPoolSetAttribute(pool, used_high, C.byref(value)) == 0  # 0 resets it
+    assert cu.cuMemPoolGetAttribute(pool, used_now, C.byref(value)) == 0
+    before = value.value
+    gpu.Graph.from_coo(u, v, opts(gpu)).close()
+    assert cu.cuMemPoolGetAttribute(pool, used_high, C.byref(value)) == 0
+    return value.value - before
+
+
+@pytest.mark.parametrize("shape", ["edges", "path", "gnp4", "gnp16", "rmat"])
+def test_memory_of_a_graph_build(gpu, shape):
+    """A build stays inside what the server sets aside for a request: 96 bytes a
+    pair, 40 a vertex at most, 8 a label."""
+    i = np.arange(2_000_000, dtype=np.uint32)
+    u, v = {"edges": lambda: (2 * i, 2 * i + 1), "path": lambda: (i, i + 1),
+            "gnp4": lambda: gpu.gen_gnp(1_000_000, 4.0, 1), "gnp16": lambda: gpu.gen_gnp(250_000, 16.0, 1),
+            "rmat": lambda: gpu.gen_rmat(17, 16, 1)}[shape]()
+    span = int(max(u.max(), v.max())) + 1
+    assert used_at_most(gpu, u, v) < 96 * len(u) + 40 * min(span, 2 * len(u)) + 8 * span + (1 << 20)
