@@ -112,3 +112,19 @@ def test_memory_of_a_graph_build(gpu, shape):
             "rmat": lambda: gpu.gen_rmat(17, 16, 1)}[shape]()
     span = int(max(u.max(), v.max())) + 1
     assert used_at_most(gpu, u, v) < 96 * len(u) + 40 * min(span, 2 * len(u)) + 8 * span + (1 << 20)
+
+
+def test_server_keeps_requests_of_many_vertices_apart(gpu):
+    """Two requests of separate edges, two vertices a pair, under a budget that
+    holds one of them: the second waits for the first."""
+    i = np.arange(1_000_000, dtype=np.uint32)
+    one = (96 + 16) * len(i) + (65 << 20)  # without the memory of the vertices
+    s = gpu.Server(memory_budget=2 * one)
+    try:
+        ids = [s.submit(2 * i, 2 * i + 1) for _ in range(2)]
+        s.drain()
+        assert all(s.poll(k)[0].count == len(i) for k in ids)
+        spans = sorted(s.span(k) for k in ids)
+    finally:
+        s.close()
+    assert spans[0][1] <= spans[1][0], spans
