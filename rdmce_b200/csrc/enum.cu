@@ -90,7 +90,7 @@ constexpr uint32_t kVertexSingles = 8;
 #define MCE_SMALL_P 9
 #endif
 constexpr int kSmallP = MCE_SMALL_P;
-static_assert(kSmallP >= 5 && kSmallP <= 12, "small-node decisions: groups double with each candidate");
+static_assert(kSmallP >= 6 && kSmallP <= 12, "t0_batch has an array of the kSmallP - 5 group candidates; groups double with each");
 // phases of the per-warp cycle accounting
 // (kCycReg: the 64-bit tier; kCycT0: the 32-bit tier)
 enum { kCycBuild = 0, kCycReg = 1, kCycGen = 2, kCycSpawn = 3, kCycIdle = 4, kCycQueue = 5, kCycT0 = 6, kCycPhases = 7 };

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const uint64_t *key
   hist[(uint64_t)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
 }
 
-// Lanes with the same digit (kRadix: no key).  Eight ballots and a select each:
+// Lanes with the same digit, among those with a key or those without.  Eight ballots and a select each:
 // match.any is one slow instruction here and bounded the whole sort.
 // Measured (B200), one pass over 16.8 M keys: 270 -> 140 us,
 // 103 us with the register bound below.
