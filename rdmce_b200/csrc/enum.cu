@@ -83,6 +83,8 @@ constexpr uint32_t kShareMin = 128, kShareMax = 8192;
 // A graph with more vertices than this for each warp has the others' small
 // vertices decided up front, 32 to a warp (tiny.cu); the late-peeled ones, up
 // to this many, are items in order either way.
+// Measured (B200), ms, for 1, 8, 32: Chung-Lu 10^6 6.89, 6.77, 6.73, R-MAT 18 of
+// edge factor 4 11.03, 10.88, 11.10, G(10^6, mean degree 6) 0.23, 0.30, 0.59.
 constexpr uint32_t kVertexSingles = 8;
 // 32-bit-tier nodes with up to this many candidates are decided in one step,
 // at 2^(n - 5) groups of about 12 instructions each (t0_small_sets).
@@ -758,6 +760,9 @@ __device__ __noinline__ void t0_batch(const EnumParams *Pm, WarpSmem *sm, uint32
 
 // A subproblem that collected fewer small nodes than this decides them one at
 // a time: a batch costs as much for one node as for 32.
+// Measured (B200), ms, for limits of 1, 8, 16, 24 and 33 (only full batches):
+// G(1000, mean degree 200) 6.32, 5.65, 5.64, 5.60, 5.62; 300 G(n, p) graphs 10.7,
+// 9.5, 9.4, 9.4, 9.4; full R-MAT 15 222, 220, 220, 223, 227.
 constexpr uint32_t kBatchMin = 16;
 
 // ------------------------------------------------ join decomposition
@@ -2382,7 +2387,10 @@ __device__ uint32_t build_rows(const DevGraph &g, const uint32_t *cand, uint32_t
       }
     }
     for (uint32_t w = lane; w < nb * W; w += 32) acc[w] = 0;
-    // probing costs p searches of a warp's lanes, reading the part len / 32 loads
+    // probing costs p searches of a warp's lanes, reading the part len / 32 loads.
+    // Measured (B200), ms, for 2, 8, 32 times p and never: 1024 core roots of
+    // R-MAT 20 27.4, 32.4, 31.7, 30.9, planted cliques of 40-200 vertices 7.15,
+    // 7.50, 7.46, 7.38; R-MAT 14, Chung-Lu 10^6 and 300 G(n, p) graphs the same
     const bool probe = len > 8 * p + 64;
     const uint32_t sl = probe ? 0 : len;
     uint32_t incl = sl;
@@ -2609,6 +2617,17 @@ __device__ bool solve_root(const Ctx &c, uint64_t r) {
 // vertex's ego network is built once and searched with a pivot;
 // from 65 later neighbours on (the general tier) only where at most
 // kVertexBranches of them, and at most a quarter, are left to branch on.
+// Measured (B200), ms:
+//   kVertexCols          64    128    256    512
+//   planted 40-200    208.4  120.4    7.5    7.8
+//   full R-MAT 14      25.2   18.9   18.8   18.4
+//   G(4000, deg 400)   34.0   33.9   35.2   38.7
+// kVertexBranches 4, 8, 16, 64: planted 16.4, 12.1, 7.5, 6.4, the others the
+// same.  An eighth, a quarter or half of them: planted 8.8, 7.5, 7.5.  Without
+// either bound planted 5.6, but G(4000, deg 400) 44.9 and G(1000, deg 200) 11.1
+// instead of 5.7.  A vertex turned down has its rows built for nothing: none on
+// R-MAT 14 and 15, 0.6 % of the warps' cycles on planted, 0.8 % on R-MAT 18 of
+// edge factor 4, 2.1 % on G(1000, 200) and G(4000, 400).
 constexpr uint32_t kVertexCols = 256, kVertexDegree = 4096, kVertexBranches = 16;
 
 // Vertex item k of the vertex pass: the cliques whose first vertex (in the
