@@ -166,7 +166,8 @@ struct WarpSmem {
   uint32_t hcache[kHistCache];
   // result accumulators for the current slot
   unsigned long long count, checksum, nodes, wops, bbytes;
-  uint32_t max_size, slot, pending, pad;
+  uint32_t max_size, slot, pending;
+  uint32_t last, singles;  // vertex pass: range_last, range_singles
   unsigned long long cyc[kCycPhases];  // clock64 cycles by phase
   // The tiers enclosing the running subproblem.  A nested tier exposes their
   // open levels (shallower, so larger) before its own: the running
@@ -2643,8 +2644,8 @@ __device__ __noinline__ uint32_t run_vertex(Ctx c, uint64_t k) {
   const EnumParams &P = *c.P;
   const DevGraph &g = P.g;
   // late-peeled vertices first: they are the heavy ones
-  const uint32_t singles = range_singles(P);
-  const uint32_t v = k < singles ? range_last(P) - (uint32_t)k : P.vert_list[k - singles];
+  const uint32_t singles = c.sm->singles;
+  const uint32_t v = k < singles ? c.sm->last - (uint32_t)k : P.vert_list[k - singles];
   const uint32_t r0 = g.root_off[v], r1 = g.root_off[v + 1];
   const uint32_t lo = (uint32_t)max((uint64_t)r0, P.rb), hi = (uint32_t)min((uint64_t)r1, P.re);
   if (lo >= hi) return 0;
@@ -2869,6 +2870,10 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
     sm->max_size = sm->slot = sm->pending = 0;
     sm->nest = 0;
     sm->share_period = kShareMin;
+    if (P.vertex_pass) {
+      sm->last = range_last(P);
+      sm->singles = range_singles(P);
+    }
   }
   sm->lchk[c.lane] = 0;
   if (c.lane == 0) {
@@ -2884,7 +2889,7 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
   c.sharing = P.sharing != 0;
   if (P.edge_list && !P.heavy_list && *P.edge_n == 0) return;  // the vertex pass left nothing (all blocks agree)
   const uint64_t total = P.heavy_list    ? P.n_heavy
-                         : P.vertex_pass ? range_singles(P) + (uint64_t)(P.vert_list ? *P.vert_n : 0)
+                         : P.vertex_pass ? sm->singles + (uint64_t)(P.vert_list ? *P.vert_n : 0)
                          : P.edge_list   ? *P.edge_n
                          : P.root_list   ? P.n_list
                                          : P.re - P.rb;
