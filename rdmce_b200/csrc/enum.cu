@@ -2618,7 +2618,7 @@ __device__ bool solve_root(const Ctx &c, uint64_t r) {
 // vertex's ego network is built once and searched with a pivot;
 // from 65 later neighbours on (the general tier) only where at most
 // kVertexBranches of them, and at most a quarter, are left to branch on.
-// Measured (B200), ms:
+// Measured (B200), ms, the G(n, p) graphs before vertices_first sent them root by root:
 //   kVertexCols          64    128    256    512
 //   planted 40-200    208.4  120.4    7.5    7.8
 //   full R-MAT 14      25.2   18.9   18.8   18.4
@@ -3010,6 +3010,27 @@ EnumParams edge_pass(const EnumPlan &plan) {
   return P;
 }
 
+// Whether a range of a graph goes vertex by vertex first.  One warp solves all
+// roots of a vertex: it takes longer than the longest root, and the roots left
+// wait for the pass to end.  So root by root, every root work of its own, where
+//   * warps outnumber the roots, or the vertices two to one;
+//   * vertices have many later neighbours on average: without a good pivot
+//     their ego networks are searched no faster than their roots', and from 65
+//     on built for nothing;
+//   * nobody takes over a heavy vertex's open work (no sharing) and there may
+//     be some.
+// Measured (B200), enumeration, ms, vertices first and root by root (4736 warps):
+//   G(64, mean degree 32) 0.128, 0.077; G(500, 64) 0.43, 0.13
+//   G(3000, 32) 0.091, 0.118; G(3000, 64) 0.46, 0.26; G(6000, 64) 0.36, 0.39
+//   G(6000, 100) 1.20, 0.82; G(30000, 64) 0.69, 1.30; G(30000, 100) 2.75, 2.29
+//   R-MAT 12 and 13, edge factor 16: 1.82, 1.91 and 3.4, 4.1
+//   without sharing: R-MAT 13 160, 45; G(200, 100) 2.7, 0.85; planted cliques of
+//   10-60 in 20,000 vertices 0.14, 0.47
+bool vertices_first(const DeviceGraph &g, uint64_t nwork, uint64_t nwarps, bool sharing) {
+  const uint64_t n = g.n, later = n < nwarps ? 24 : 40;
+  return nwork > nwarps && 2 * n >= nwarps && g.m <= later * n && (sharing || g.max_degree <= 256);
+}
+
 }  // namespace
 
 mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, Scratch *scr, SlotResult *slots,
@@ -3105,7 +3126,7 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   if (!slab) return s;
   // A range goes vertex by vertex first; per-root values and the counters of
   // the edge-rooted method (stats) need every root on its own.
-  plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && nwork;
+  plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && vertices_first(g, nwork, nwarps, P.sharing);
   // One buffer of lists: the vertex pass's roots and vertices left, and the
   // roots whose ego network overflows the slab, deferred to a second pass.
   // Those are kept by work index (a solve of more than 2^32 roots is refused by
