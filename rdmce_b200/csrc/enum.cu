@@ -2205,14 +2205,16 @@ __device__ __forceinline__ uint32_t window_for(const uint32_t *b, uint32_t n, ui
 // Bound by the latency of the searches in the longer list, so four of the
 // shorter list's 32-element groups are searched at a time, and where the lists
 // are long and of like lengths only in the part of the longer one that the
-// groups span (a few cache lines instead of the whole list).
+// groups span (a few cache lines instead of the whole list).  Lists of up to 512
+// are found faster whole: G(12000, mean degree 150) 2.99 ms instead of 3.14,
+// G(4000, 400) 31.9 instead of 33.0 (B200).
 __device__ uint32_t intersect(const DevGraph &g, uint32_t v0, uint32_t v1, uint32_t *cand, uint64_t cap) {
   const uint32_t lane = lane_id();
   const uint32_t *a, *b;
   uint32_t da, db;
   shorter_first(g, v0, v1, a, da, b, db);
   uint32_t nc = 0;
-  const bool windows = da > 128 && db / 64 < da;
+  const bool windows = da > 128 && db > 512 && db / 64 < da;
   uint32_t done = 0;  // elements of b below every value still to come
   for (uint32_t base = 0; base < da; base += 128) {
     uint32_t val[4];
