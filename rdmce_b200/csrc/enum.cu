@@ -3018,18 +3018,24 @@ EnumParams edge_pass(const EnumPlan &plan) {
 //   * warps outnumber the roots, or the vertices two to one;
 //   * vertices have many later neighbours on average: without a good pivot
 //     their ego networks are searched no faster than their roots', and from 65
-//     on built for nothing;
+//     on built for nothing -- unless the mean vertex is adjacent to a sixth of
+//     its graph (the graphs are many then), where a vertex's roots share most
+//     of their networks;
 //   * nobody takes over a heavy vertex's open work (no sharing) and there may
 //     be some.
 // Measured (B200), enumeration, ms, vertices first and root by root (4736 warps):
 //   G(64, mean degree 32) 0.128, 0.077; G(500, 64) 0.43, 0.13
 //   G(3000, 32) 0.091, 0.118; G(3000, 64) 0.46, 0.26; G(6000, 64) 0.36, 0.39
 //   G(6000, 100) 1.20, 0.82; G(30000, 64) 0.69, 1.30; G(30000, 100) 2.75, 2.29
+//   100 x G(300, 90) 13.6, 19.0; 40 x G(500, 100) 8.1, 8.6; 30 x G(1000, 100) 8.3,
+//   8.4; 60 x G(1000, 150) 58, 49
 //   R-MAT 12 and 13, edge factor 16: 1.82, 1.91 and 3.4, 4.1
 //   without sharing: R-MAT 13 160, 45; G(200, 100) 2.7, 0.85; planted cliques of
 //   10-60 in 20,000 vertices 0.14, 0.47
-bool vertices_first(const DeviceGraph &g, uint64_t nwork, uint64_t nwarps, bool sharing) {
-  const uint64_t n = g.n, later = n < nwarps ? 24 : 40;
+bool vertices_first(const DeviceGraph &g, uint64_t nwork, uint64_t nwarps, uint64_t n_graphs, bool sharing) {
+  const uint64_t n = g.n;
+  const bool dense = 12 * g.m * n_graphs >= n * n;
+  const uint64_t later = n < nwarps ? 24 : dense ? 256 : 40;
   return nwork > nwarps && 2 * n >= nwarps && g.m <= later * n && (sharing || g.max_degree <= 256);
 }
 
@@ -3128,7 +3134,7 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   if (!slab) return s;
   // A range goes vertex by vertex first; per-root values and the counters of
   // the edge-rooted method (stats) need every root on its own.
-  plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && vertices_first(g, nwork, nwarps, P.sharing);
+  plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && vertices_first(g, nwork, nwarps, cfg.n_slots, P.sharing);
   // One buffer of lists: the vertex pass's roots and vertices left, and the
   // roots whose ego network overflows the slab, deferred to a second pass.
   // Those are kept by work index (a solve of more than 2^32 roots is refused by

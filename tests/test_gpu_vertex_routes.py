@@ -53,3 +53,21 @@ def test_full_solve_is_not_slower_than_its_roots(gpu, name, sharing):
     assert {(r.count, r.checksum) for r in full} == {(r.count, r.checksum) for r in each}
     full_ms, each_ms = (min(r.phase_ms[3] for r in rs) for rs in (full, each))
     assert full_ms < 1.4 * each_ms, (full_ms, each_ms)
+
+
+def test_batch_of_dense_graphs_is_faster_than_its_roots(gpu):
+    """Graphs whose mean vertex is adjacent to a third of its graph: a vertex's
+    roots share most of their ego networks."""
+    graphs = [gpu.gen_gnp(300, 90.0, i) for i in range(100)]
+    o = opts(gpu, blocks_per_sm=4)
+    b = gpu.Batch(graphs, opts(gpu))
+    try:
+        full = [b.solve(o) for _ in range(5)]
+    finally:
+        b.close()
+    u, v = (np.concatenate([g[k] + 300 * i for i, g in enumerate(graphs)]).astype(np.uint32) for k in (0, 1))
+    with gpu.Graph.from_coo(u, v, opts(gpu)) as g:
+        roots = np.arange(g.info()["num_edges"], dtype=np.uint64)
+        each = [g.solve_root_list(roots, o) for _ in range(5)]
+    assert sum(r["count"] for r in full[-1][0]) == each[-1].count
+    assert min(r[2] for r in full[1:]) < 0.9 * min(r.phase_ms[3] for r in each[1:])
