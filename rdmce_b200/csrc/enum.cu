@@ -372,8 +372,8 @@ __device__ __forceinline__ void pool_publish(const Ctx &c, uint32_t blk) {
   __threadfence();
   __syncwarp();
   if (c.lane == 0) {
-    atomicAdd(P.active, 1u);
     __threadfence();
+    atomicAdd(P.active, 1u);  // ordered before the task by ring_push's fence
     if (!ring_push(P.ready_slot, P.ready_seq, P.ready_tail, P.ready_count, P.pool_mask, blk, P)) atomicSub(P.active, 1u);
     atomicAdd(P.stat_tasks, 1ULL);
   }
@@ -2804,7 +2804,7 @@ __device__ __noinline__ void run_root(Ctx c, uint64_t k) {
 // At most one warp per block polls the global queue at a time (the block's
 // poll token); the others sleep.  The busy count holds every warp that may
 // still claim an item and every task from before it is published until its
-// taker has finished it.  Whoever adds to it is counted already (a task's
+// taker, unless that counts itself, has finished it.  Whoever adds to it is counted already (a task's
 // producer; a warp before its first claim), so zero in this one word means that
 // no task is queued or held: one look is enough, in any order of the ring's
 // own counts.  (Warps that start late count themselves in, and wait for zero
@@ -2912,11 +2912,10 @@ __global__ void __launch_bounds__(256, MCE_ENUM_BPS) k_enumerate(const __grid_co
       if (c.lane == 0) sm->cyc[kCycQueue] += now() - tq;
       if (got) {
         const unsigned long long tb = now();
+        // this warp counts itself; two for one busy warp would hide an idle one
+        if (c.lane == 0) atomicSub(P.active, 1u);
         solve_block(c, blk);
-        if (c.lane == 0) {
-          atomicMax(P.stat_max_item + 1, now() - tb);
-          atomicSub(P.active, 1u);
-        }
+        if (c.lane == 0) atomicMax(P.stat_max_item + 1, now() - tb);
         continue;
       }
     }
