@@ -136,6 +136,10 @@ struct SlotResult {
 struct Scratch;
 
 // Kernel parameters of one enumeration launch.
+// Which vertices of a range are solved whole before the roots that are left:
+// none, those with a good pivot, all that are not too large.
+enum VertexPass : int { kNoVertices = 0, kPivotVertices = 1, kAllVertices = 2 };
+
 struct EnumParams {
   DevGraph g;
   uint64_t rb, re;                       // root range [rb, re) (range mode)
@@ -143,7 +147,7 @@ struct EnumParams {
   uint64_t n_heavy;                      // entries in heavy_list
   const uint64_t *root_list;             // list mode: root ids (else the range [rb, re))
   uint64_t n_list;                       // entries in root_list
-  int vertex_pass;                       // work items are the vertices of the range, not its roots
+  int vertex_pass;                       // a VertexPass: work items are the vertices of the range, not its roots
   uint32_t *vert_list;                   // vertex pass: of the vertices before the graph's last single_items, those to take (null: all)
   uint64_t single_items;
   unsigned int *vert_n;                  // how many

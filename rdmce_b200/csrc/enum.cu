@@ -2633,6 +2633,71 @@ __device__ bool solve_root(const Ctx &c, uint64_t r) {
 // edge factor 4, 2.1 % on G(1000, 200) and G(4000, 400).
 constexpr uint32_t kVertexCols = 256, kVertexDegree = 4096, kVertexBranches = 16;
 
+// Whether val is in each of four sorted lists, searched in step.
+__device__ __forceinline__ void contains_each(const uint32_t *const (&list)[4], const uint32_t (&n)[4], uint32_t val,
+                                              bool (&hit)[4]) {
+  uint32_t pos[4] = {0, 0, 0, 0}, len[4] = {n[0], n[1], n[2], n[3]};
+  while (max(max(len[0], len[1]), max(len[2], len[3])) > 1) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t half = len[k] >> 1;
+      if (half && __ldg(list[k] + pos[k] + half - 1) < val) pos[k] += half;
+      len[k] -= half;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) hit[k] = __ldg(list[k] + pos[k]) == val;
+}
+
+// Whether one of the four candidates Pl[0..p) of most neighbours is a pivot that
+// leaves at most kVertexBranches of them, and at most a quarter, to branch on.
+// Of the vertices with such a pivot, 96 to 100 % have one among these four
+// (R-MAT 12 to 18, Chung-Lu 10^6, planted cliques).  A sample of 32 candidates
+// turns most others down after one search.
+__device__ __noinline__ bool good_pivot(const DevGraph &g, const uint32_t *Pl, uint32_t p) {
+  if (p < 4) return false;
+  const uint32_t lane = lane_id();
+  uint32_t key[kVertexCols / 32];  // neighbours << 8 | candidate, 0: none
+#pragma unroll
+  for (int k = 0; k < (int)kVertexCols / 32; k++) {
+    const uint32_t j = 32 * k + lane;
+    key[k] = 0;
+    if (j < p) {
+      const uint32_t u = __ldg(Pl + j);
+      key[k] = min(g.off[u + 1] - g.off[u], 0xffffffu) << 8 | j;
+    }
+  }
+  const uint32_t *list[4];
+  uint32_t n[4], hits[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int t = 0; t < 4; t++) {
+    uint32_t top = 0;
+#pragma unroll
+    for (int k = 0; k < (int)kVertexCols / 32; k++) top = max(top, key[k]);
+    top = __reduce_max_sync(kFull, top);
+#pragma unroll
+    for (int k = 0; k < (int)kVertexCols / 32; k++)
+      if (key[k] == top) key[k] = 0;
+    const uint32_t u = __ldg(Pl + (top & 0xff));
+    list[t] = g.adj + g.off[u];
+    n[t] = g.off[u + 1] - g.off[u];
+  }
+  bool hit[4];
+  contains_each(list, n, __ldg(Pl + lane * p / 32), hit);
+  uint32_t best = 0;
+#pragma unroll
+  for (int t = 0; t < 4; t++) best = max(best, (uint32_t)__popc(__ballot_sync(kFull, hit[t])));
+  if (best < 16) return false;
+  for (uint32_t base = 0; base < p; base += 32) {
+    const uint32_t j = base + lane;
+    contains_each(list, n, j < p ? __ldg(Pl + j) : 0, hit);
+#pragma unroll
+    for (int t = 0; t < 4; t++) hits[t] += __popc(__ballot_sync(kFull, j < p && hit[t]));
+  }
+  const uint32_t left = p - max(max(hits[0], hits[1]), max(hits[2], hits[3]));
+  return left <= kVertexBranches && 4 * left <= p;
+}
+
 // Vertex item k of the vertex pass: the cliques whose first vertex (in the
 // order) is v.  An edge root (v, w) builds its own ego network out of the
 // members' lists, so a member's list is read once for every w it is adjacent
@@ -2654,9 +2719,10 @@ __device__ __noinline__ uint32_t run_vertex(Ctx c, uint64_t k) {
   const unsigned long long t0 = now();
   const uint32_t b = g.off[v], d = g.off[v + 1] - b, p = r1 - r0, x = d - p, W = (p + 63) / 64;
   const Layout L = layout_for(0, p, d, W);
-  bool whole = hi - lo == p && p <= kVertexCols && d <= kVertexDegree && L.need <= c.slab_bytes;
+  const uint32_t *cand = g.adj + b;
+  bool whole = hi - lo == p && p <= kVertexCols && d <= kVertexDegree && L.need <= c.slab_bytes &&
+               (P.vertex_pass != kPivotVertices || good_pivot(g, cand + x, p));
   if (whole) {
-    const uint32_t *cand = g.adj + b;
     uint64_t *rows = (uint64_t *)(c.slab + L.rows_off);
     set_slot(c, g.slot ? g.slot[v] : 0);
     const uint32_t nrows = build_rows(g, cand, x, p, W, rows, c.sm);
@@ -3011,18 +3077,23 @@ EnumParams edge_pass(const EnumPlan &plan) {
   return P;
 }
 
-// Whether a range of a graph goes vertex by vertex first.  One warp solves all
-// roots of a vertex: it takes longer than the longest root, and the roots left
-// wait for the pass to end.  So root by root, every root work of its own, where
-//   * warps outnumber the roots, or the vertices two to one;
+// How a range of a graph goes: root by root, or vertices first, all of them or
+// those with a good pivot.  One warp solves all roots of a vertex: it takes
+// longer than the longest root, and the roots left wait for the pass to end.
+// Root by root, every root work of its own, where
+//   * warps outnumber the roots;
+//   * nobody takes over a heavy vertex's open work (no sharing) and there may
+//     be some.
+// Not all vertices, where
+//   * warps outnumber the vertices two to one;
 //   * vertices have many later neighbours on average: without a good pivot
 //     their ego networks are searched no faster than their roots', and from 65
 //     on built for nothing -- unless the mean vertex is adjacent to a sixth of
 //     its graph (the graphs are many then), where a vertex's roots share most
-//     of their networks;
-//   * nobody takes over a heavy vertex's open work (no sharing) and there may
-//     be some.
-// Measured (B200), enumeration, ms, vertices first and root by root (4736 warps):
+//     of their networks.
+// Looking for pivots takes a pass of its own, which pays from ego networks of 64
+// later neighbours on.
+// Measured (B200, 4736 warps), enumeration, ms, vertices first and root by root:
 //   G(64, mean degree 32) 0.128, 0.077; G(500, 64) 0.43, 0.13
 //   G(3000, 32) 0.091, 0.118; G(3000, 64) 0.46, 0.26; G(6000, 64) 0.36, 0.39
 //   G(6000, 100) 1.20, 0.82; G(30000, 64) 0.69, 1.30; G(30000, 100) 2.75, 2.29
@@ -3031,11 +3102,16 @@ EnumParams edge_pass(const EnumPlan &plan) {
 //   R-MAT 12 and 13, edge factor 16: 1.82, 1.91 and 3.4, 4.1
 //   without sharing: R-MAT 13 160, 45; G(200, 100) 2.7, 0.85; planted cliques of
 //   10-60 in 20,000 vertices 0.14, 0.47
-bool vertices_first(const DeviceGraph &g, uint64_t nwork, uint64_t nwarps, uint64_t n_graphs, bool sharing) {
+// and with pivots only: 300 cliques of 200 vertices 17.7, 972, 17.9; G(6000, 150)
+// 3.3, 2.1, 2.1; G(3000, 64) 0.46, 0.26, 0.33.
+VertexPass vertex_pass_for(const DeviceGraph &g, uint64_t nwork, uint64_t nwarps, uint64_t n_graphs, bool sharing) {
+  if (nwork <= nwarps) return kNoVertices;
+  if (!sharing && g.max_degree > 256) return kNoVertices;
   const uint64_t n = g.n;
   const bool dense = 12 * g.m * n_graphs >= n * n;
   const uint64_t later = n < nwarps ? 24 : dense ? 256 : 40;
-  return nwork > nwarps && 2 * n >= nwarps && g.m <= later * n && (sharing || g.max_degree <= 256);
+  if (2 * n >= nwarps && g.m <= later * n) return kAllVertices;
+  return g.degeneracy < 64 || (!sharing && 2 * n < nwarps) ? kNoVertices : kPivotVertices;
 }
 
 }  // namespace
@@ -3133,7 +3209,10 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   if (!slab) return s;
   // A range goes vertex by vertex first; per-root values and the counters of
   // the edge-rooted method (stats) need every root on its own.
-  plan->vertex_pass = !list_mode && !P.per_root_count && !P.stats && vertices_first(g, nwork, nwarps, cfg.n_slots, P.sharing);
+  const VertexPass pass_kind = list_mode || P.per_root_count || P.stats
+                                   ? kNoVertices
+                                   : vertex_pass_for(g, nwork, nwarps, cfg.n_slots, P.sharing);
+  plan->vertex_pass = pass_kind != kNoVertices;
   // One buffer of lists: the vertex pass's roots and vertices left, and the
   // roots whose ego network overflows the slab, deferred to a second pass.
   // Those are kept by work index (a solve of more than 2^32 roots is refused by
@@ -3173,7 +3252,7 @@ mce_status MCE_ENUM_FN(enum_plan)(const DeviceGraph &g, const EnumConfig &cfg, S
   P.root_list = list_mode ? cfg.root_list : nullptr;
   P.n_list = list_mode ? cfg.n_root_list : 0;
   if (plan->vertex_pass) {
-    P.vertex_pass = 1;
+    P.vertex_pass = pass_kind;
     P.edge_out = heavy + heavy_cap;
     P.edge_n = &ctl->edge_n;
     if (g.n > kVertexSingles * nwarps) {

@@ -71,3 +71,23 @@ def test_batch_of_dense_graphs_is_faster_than_its_roots(gpu):
         each = [g.solve_root_list(roots, o) for _ in range(5)]
     assert sum(r["count"] for r in full[-1][0]) == each[-1].count
     assert min(r[2] for r in full[1:]) < 0.9 * min(r.phase_ms[3] for r in each[1:])
+
+
+@pytest.mark.parametrize("count,size", [(3, 200), (60, 150)])
+def test_cliques_are_solved_by_vertex(gpu, oracle_mod, count, size):
+    """Many later neighbours and a perfect pivot: such vertices are solved whole,
+    which is far faster than each of their roots where there are vertices for
+    the warps.  Cliques with some edges taken out have several maximal cliques each."""
+    i, j = np.triu_indices(size, 1)
+    keep = np.random.default_rng(size).random(len(i)) < 0.999
+    u, v = (np.concatenate([x[keep] + size * k for k in range(count)]).astype(np.uint32) for x in (i, j))
+    o = oracle_mod.Graph.from_pairs(u, v).sort_degeneracy().mce(threads=THREADS)
+    with gpu.Graph.from_coo(u, v, opts(gpu)) as g:
+        roots = np.arange(g.info()["num_edges"], dtype=np.uint64)
+        full = [g.solve(opts(gpu, blocks_per_sm=4)) for _ in range(4)]
+        each = [g.solve_root_list(roots, opts(gpu, blocks_per_sm=4)) for _ in range(4)]
+        assert_same(g.solve(opts(gpu, flags=gpu.FLAG_NO_SHARING)), o)
+    assert_same(full[-1], o)
+    assert_same(each[-1], o)
+    if count > 3:
+        assert min(r.phase_ms[3] for r in full) < 0.6 * min(r.phase_ms[3] for r in each)
