@@ -74,7 +74,7 @@ typedef struct mce_options {
   int expand_r;               /* aggressive node generation (mce_gpu.cuh:5); default 1 */
   uint64_t root_begin;        /* enumerate roots [root_begin, root_end); 0,0 = all roots */
   uint64_t root_end;
-  uint64_t spin_limit;        /* bound on every device-side wait; 0 = default */
+  uint64_t spin_limit;        /* bound on every device-side wait; 0 = default (a graph build polls 2^26 times at least) */
   void *stream;               /* cudaStream_t to run on; NULL = the engine's own stream */
   uint32_t flags;             /* MCE_FLAG_* */
   uint32_t reg_share_bound;   /* tau inside the register tiers (<= 64 columns); 0 = 24, never above share_bound */
