@@ -2620,7 +2620,7 @@ __device__ bool solve_root(const Ctx &c, uint64_t r) {
 // vertex's ego network is built once and searched with a pivot;
 // from 65 later neighbours on (the general tier) only where at most
 // kVertexBranches of them, and at most a quarter, are left to branch on.
-// Measured (B200), ms, the G(n, p) graphs before vertices_first sent them root by root:
+// Measured (B200), ms, with all vertices of the G(n, p) graphs first (vertex_pass_for):
 //   kVertexCols          64    128    256    512
 //   planted 40-200    208.4  120.4    7.5    7.8
 //   full R-MAT 14      25.2   18.9   18.8   18.4
